@@ -195,7 +195,7 @@ KC_HD double clear_lo_word(double x) { return from_bits(to_bits(x) & 0xffffffff0
 
 // exp: x = k ln2 + r with ln2 split in two (k ln2hi exact), |r| <= ln2/2;
 // e^r from the Remez rational form 1 + r + r c(r) / (2 - c(r)), then 2^k.
-KC_HDN double exp(double x) {
+KC_HD double exp_inl(double x) {
   const double ln2hi = 6.93147180369123816490e-01, ln2lo = 1.90821492927058770002e-10,
                invln2 = 1.44269504088896338700e+00;
   const double P1 = 1.66666666666666019037e-01, P2 = -2.77777777770155933842e-03,
@@ -230,8 +230,12 @@ KC_HDN double exp(double x) {
   const double xx = x * x;
   const double c = x - xx * (P1 + xx * (P2 + xx * (P3 + xx * (P4 + xx * P5))));
   const double y = 1.0 + (x * c / (2.0 - c) - lo + hi);
-  return k == 0 ? y : ldexp(y, k);
+  if (k == 0) return y;
+  // ldexp's own product for every k of a normal result, its rescaling loops aside
+  if (k >= -1022 && k <= 1023) return y * from_bits((uint64_t)(k + 1023) << 52);
+  return ldexp(y, k);
 }
+KC_HDN double exp(double x) { return exp_inl(x); }
 
 // ---- log -------------------------------------------------------------------
 // Tang's table-driven logarithm. Both reference scenarios that pin the Zig
@@ -257,7 +261,7 @@ KC_HD double log_core(int k, double m) {
   return s2 + (e1 + e2 + ((dk * KM_LN2_LO + llo) + lo));
 }
 
-KC_HDN double log(double x) {
+KC_HD double log_inl(double x) {
   if (x != x) return x;
   if (x < 0.0) return nan();
   if (x == 0.0) return -inf();
@@ -276,11 +280,12 @@ KC_HDN double log(double x) {
   }
   return log_core(k + e, m);
 }
+KC_HDN double log(double x) { return log_inl(x); }
 
 // log1p: u = 1 + x = 2^k (1 + f) with 1 + f in [sqrt(2)/2, sqrt(2)), the
 // rounding of u carried as c/u; log(1+f) = f - f^2/2 + s (f^2/2 + R(s^2)),
 // s = f / (2 + f), R the fdlibm Lg1..Lg7 polynomial.
-KC_HDN double log1p(double x) {
+KC_HD double log1p_inl(double x) {
   const double ln2_hi = 6.93147180369123816490e-01, ln2_lo = 1.90821492927058770002e-10;
   const double Lg1 = 6.666666666666735130e-01, Lg2 = 3.999999999940941908e-01, Lg3 = 2.857142874366239149e-01,
                Lg4 = 2.222219843214978396e-01, Lg5 = 1.818357216161805012e-01, Lg6 = 1.531383769920937332e-01,
@@ -320,11 +325,12 @@ KC_HDN double log1p(double x) {
   const double dk = (double)k;
   return s * (hfsq + (t2 + t1)) + (dk * ln2_lo + c) - hfsq + f + dk * ln2_hi;
 }
+KC_HDN double log1p(double x) { return log1p_inl(x); }
 
 // ---- cbrt ------------------------------------------------------------------
 // Seed from the exponent divided by three, a polynomial step to ~23 bits,
 // rounding to 22 bits (so t*t is exact), one Newton-like step in double.
-KC_HDN double cbrt(double x) {
+KC_HD double cbrt_inl(double x) {
   const uint32_t B1 = 715094163, B2 = 696219795;
   const double P0 = 1.87595182427177009643, P1 = -1.88497979543377169875, P2 = 1.621429720105354466140,
                P3 = -0.758397934778766047437, P4 = 0.145996192886612446982;
@@ -349,6 +355,7 @@ KC_HDN double cbrt(double x) {
   r = (r - t) / (w + r);
   return t + t * r;
 }
+KC_HDN double cbrt(double x) { return cbrt_inl(x); }
 
 // ---- trigonometric ---------------------------------------------------------
 // Kernels on |x| <= pi/4 with the reduced argument's tail y.

@@ -62,6 +62,7 @@ struct kc_handle {
   // step scalars (koral/sim.zig:237-293)
   double t = 0, dt = 0, own_dt = 0, tstepdenmax = 0, tstepdenmin = 1.0e50;
   double min_dx = 0, min_dy = 0, min_dz = 0;
+  int nsm = 1;          // SMs of the device
   int impl_blocks = 0;  // resident blocks of the persistent implicit kernel
   double* init_dv = nullptr;  // the PUFFY init's per-column torus profile
   // block sizes of the per-cell implicit, face-flux and u2p kernels (kc_autotune);
@@ -394,6 +395,16 @@ int ensure_split(kc_handle* h) {
   return KC_OK;
 }
 
+// Cells that each warp of the implicit pass carries: all 32 lanes once the grid has
+// 32 cells for four warps an SM, fewer on smaller grids, whose passes last as long
+// as their slowest warp (the union of its lanes' paths; one solve is a serial
+// chain of dependent FP64 operations either way). Measured, ladder per launch:
+// 32x30 171 us with 32, 156 with 2 to 8, 162 with 1; 32x30x4 210 with 32, 179 with
+// 4, 291 with 2; 101x75 187 with 32, 189 with 16, 286 with 4.
+int implicit_lanes(long ncell, int nsm) {
+  const long l = (ncell + 4L * nsm - 1) / (4L * nsm);
+  return l > 32 ? 32 : (int)l;
+}
 void launch_implicit(kc_handle* h, int dt_slot) {
   const DGrid& gr = h->gr;
   ImplArgs a;
@@ -453,16 +464,26 @@ void launch_implicit(kc_handle* h, int dt_slot) {
     k_mlp_guess<<<nblk(ndom), TPB, 0, h->stream>>>(h->ds, m, a, h->guess);
     x.guess = h->guess;
   }
-  ++h->n_launch;
-  // one block per SM; the learned-guess and harvest forms in the default block
-  const int nt = extra || (h->tpb_implicit != 256 && h->tpb_implicit != 512) ? KC_IMPLICIT_TPB : h->tpb_implicit;
-  const unsigned nb = nblk(ndom, nt);
   cudaStream_t st = h->stream;
-  if (h->hcap > 0) k_implicit<IMPL_FULL, KC_IMPLICIT_TPB><<<nb, nt, 0, st>>>(h->ds, h->dsc, a, x);
-  else if (extra) k_implicit<IMPL_GUESS, KC_IMPLICIT_TPB><<<nb, nt, 0, st>>>(h->ds, h->dsc, a, x);
-  else if (nt == 256) k_implicit<IMPL_PLAIN, 256><<<nb, nt, 0, st>>>(h->ds, h->dsc, a, x);
-  else if (nt == 512) k_implicit<IMPL_PLAIN, 512><<<nb, nt, 0, st>>>(h->ds, h->dsc, a, x);
-  else k_implicit<IMPL_PLAIN, KC_IMPLICIT_TPB><<<nb, nt, 0, st>>>(h->ds, h->dsc, a, x);
+  // the AoS staging array is free inside a step: 8 doubles and an int per cell of its NV doubles
+  const WarmBuf wb = {h->staging, (int*)(h->staging + 8 * ndom), ndom};
+  const int lanes = implicit_lanes(ndom, h->nsm);
+  const long nthread = (ndom + lanes - 1) / lanes * 32;
+  h->n_launch += 2;
+  if (x.guess)
+    k_implicit_pick<<<nblk(nthread, KC_PICK_TPB), KC_PICK_TPB, SharedCell::bytes(KC_PICK_TPB), st>>>(h->ds, h->dsc, a, wb,
+                                                                                                    x.guess, lanes);
+  else
+    k_implicit_warm<<<nblk(nthread, KC_WARM_TPB), KC_WARM_TPB, 0, st>>>(h->ds, a, wb, lanes);
+  // the learned-guess and harvest forms in the default block
+  const int nt = extra ? KC_IMPLICIT_TPB : h->tpb_implicit;
+  const unsigned nb = nblk(nthread, nt);
+  const size_t sm = SharedCell::bytes(nt);
+  if (h->hcap > 0) k_implicit_ext<true><<<nb, nt, sm, st>>>(h->ds, h->dsc, a, wb, x, lanes);
+  else if (extra) k_implicit_ext<false><<<nb, nt, sm, st>>>(h->ds, h->dsc, a, wb, x, lanes);
+  else if (nt == 256) k_implicit<256><<<nb, nt, sm, st>>>(h->ds, h->dsc, a, wb, lanes);
+  else if (nt == 512) k_implicit<512><<<nb, nt, sm, st>>>(h->ds, h->dsc, a, wb, lanes);
+  else k_implicit<384><<<nb, nt, sm, st>>>(h->ds, h->dsc, a, wb, lanes);
 }
 
 void launch_wavespeeds(kc_handle* h) {
@@ -882,6 +903,7 @@ int kc_create(const kc_grid* grid, const kc_options* opt, kc_handle** out) {
   if (opt->device < 0 || opt->device >= ndev) return fail(h, KC_ERR_INVALID_CONFIG, "device ordinal out of range");
   int st = cuda_check(h, cudaSetDevice(opt->device), "cudaSetDevice");
   if (st) return st;
+  cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, opt->device);
   st = cuda_check(h, cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "cudaStreamCreate");
   if (st) return st;
   // the tiled face kernels stage more than the default 48 KB of shared memory
@@ -889,6 +911,17 @@ int kc_create(const kc_grid* grid, const kc_options* opt, kc_handle** out) {
                                           (int)sizeof(FaceTile)), "face tile shared memory");
   if (!st) st = cuda_check(h, cudaFuncSetAttribute(k_face_flux_tiled<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    (int)sizeof(FaceTile)), "face tile shared memory");
+  // the implicit kernels hold their cells in shared memory
+  const auto smem = [&](const void* f, int threads) {
+    return cuda_check(h, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SharedCell::bytes(threads)),
+                      "implicit shared memory");
+  };
+  if (!st) st = smem((const void*)k_implicit<256>, 256);
+  if (!st) st = smem((const void*)k_implicit<384>, 384);
+  if (!st) st = smem((const void*)k_implicit<512>, 512);
+  if (!st) st = smem((const void*)k_implicit_pick, KC_PICK_TPB);
+  if (!st) st = smem((const void*)k_implicit_ext<false>, KC_IMPLICIT_TPB);
+  if (!st) st = smem((const void*)k_implicit_ext<true>, KC_IMPLICIT_TPB);
   if (st) return st;
   Grid g = grid_init(grid->nx, grid->ny, grid->nz, grid->ng, grid->minx, grid->maxx, grid->miny, grid->maxy, grid->minz,
                      grid->maxz);

@@ -5,6 +5,7 @@
 // (--fmad=false) reproduces the CPU oracle bit for bit.
 #pragma once
 #include "kc_dev.cuh"
+#include "kc_implicit_lean.cuh"
 #include "kc_implicit_sm.cuh"
 #include "kc_mixed.cuh"
 #include "kc_mlp.cuh"
@@ -22,6 +23,13 @@
 #endif
 #ifndef KC_DYNAMO_MIN_BLOCKS
 #define KC_DYNAMO_MIN_BLOCKS 3
+#endif
+// Threads per block and resident blocks of the warm-start kernel
+#ifndef KC_WARM_TPB
+#define KC_WARM_TPB 128
+#endif
+#ifndef KC_WARM_MIN_BLOCKS
+#define KC_WARM_MIN_BLOCKS 4
 #endif
 #ifndef KC_BC_MIN_BLOCKS
 #define KC_BC_MIN_BLOCKS 1
@@ -1176,105 +1184,358 @@ __device__ __noinline__ bool presolve_needs_newton(const double pp00[NV], const 
   const double e0 = implicit_start_residual(uu00, st00, pp00, g, dt, a.gam, a.rp, a.op, 1.0, a.ip, sw, pc);
   return !(e0 < a.ip.conv);
 }
-// FORM: IMPL_PLAIN is the reference path alone (the guess and harvest code is
-// not compiled into it, so its registers and code size are those of the plain
-// solve); IMPL_GUESS adds the learned start only; IMPL_FULL the learned start
-// and the training-pair harvest.
-// NT: threads per block, and one block per SM: the register budget follows
-// (256 threads: 255 registers, 8 warps; 384: 168, 12 warps; 512: 128, 16 warps;
-// an SM sub-partition holds 16 K registers, so no budget between these gives
-// more warps). Every form runs in two block-synchronous phases: every thread's
-// warm start (the 1-D bisection, or the learned start's pick), a block barrier,
-// then every thread's ladder, so that all warps of the SM execute the same part
-// of the solver's code at a time (the code is far larger than the instruction
-// cache). Measured on the 192x180x64 wedge, implicit pass per step: one
-// unsynchronised pass in blocks of 128 58.1 ms (255 registers, 2 blocks per SM);
-// the two phases in blocks of 128 56.4; SM-wide blocks of 256 50.2, of 384 46.0,
-// of 512 48.2; a third phase (the rung-0 first residual test) 52.9 at 256.
-enum : int { IMPL_PLAIN = 0, IMPL_GUESS = 1, IMPL_FULL = 2 };
-#ifndef KC_IMPLICIT_TPB
-#define KC_IMPLICIT_TPB 384  // the default block: 12 warps, 168 registers
-#endif
-template <int FORM, int NT>
-__global__ void __launch_bounds__(NT, 1) k_implicit(DevState s, DevScalars* sc, const __grid_constant__ ImplArgs a,
-                                                        ImplExtra x) {
-  const double dt = s.coef[a.dt_slot];
-  long ix = 0, iy = 0, iz = 0;
-  bool act;
+// The domain cell of this thread in the implicit pass's order; false past the
+// end and in the polar band. td: the thread's index.
+__device__ __forceinline__ bool implicit_cell(const DGrid& gr, const ImplArgs& a, long t, long& ix, long& iy, long& iz) {
+  if (t >= (long)gr.nx * gr.ny * gr.nz) return false;
   if (a.phi_fastest) {
-    act = domain_cell_phi_fastest(s.gr, ix, iy, iz);
+    iz = t % gr.nz;
+    const long q = t / gr.nz;
+    ix = q % gr.nx;
+    iy = q / gr.nx;
   } else if (a.y_fastest) {
     // 2D: neighbours in theta at one radius (measured 10% faster than x fastest
     // on the 384x360 grid; 8 x 4 tiles per warp were in between)
-    long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    act = t < (long)s.gr.nx * s.gr.ny * s.gr.nz;
-    if (act) {
-      iy = t % s.gr.ny;
-      long q = t / s.gr.ny;
-      ix = q % s.gr.nx;
-      iz = q / s.gr.nx;
-    }
+    iy = t % gr.ny;
+    const long q = t / gr.ny;
+    ix = q % gr.nx;
+    iz = q / gr.nx;
   } else {
-    Range r = {0, 0, 0, s.gr.nx, s.gr.ny, s.gr.nz};
-    act = range_cell(r, ix, iy, iz);
+    ix = t % gr.nx;
+    const long q = t / gr.nx;
+    iy = q % gr.ny;
+    iz = q / gr.ny;
   }
-  if (act && a.polar_nc > 0 && (iy < a.polar_nc || iy > s.gr.ny - a.polar_nc - 1)) act = false;
-  long nc = s.gr.nc, c = act ? cidx(s.gr, ix, iy, iz) : 0;
-  constexpr bool HARVEST = FORM == IMPL_FULL;
-  const bool guessed = FORM != IMPL_PLAIN && x.guess != nullptr;
-  // the cell's metric is read once and its state written once: evict-first in
-  // L2 (which keeps L2 for the solver's call frames); the state loads stay plain
-  // (their evict-first form costs the kernel registers and 200 bytes of spills)
-  double uu[NV], pp[NV], pp00[NV];
+  return !(a.polar_nc > 0 && (iy < a.polar_nc || iy > gr.ny - a.polar_nc - 1));
+}
+// The warm starts of a pass, by thread index: energies of the start state, the
+// reference state's radiation energy and the start fluid.
+struct WarmBuf {
+  double* v;  // [8][n]: uu, ee, ehat, conserved entropy and, for lag_opac, the reference state's four opacities
+  int* startwith;
+  long n;
+};
+// The bisection warm start of every cell: a loop of one slim residual whose
+// constants stay in registers (kc_implicit_lean.cuh). Bound by dependent FP64
+// latency at half of the issue slots and 45% of the FP64 pipe; 1.33 ms a launch
+// on the 192x180x64 wedge (as the first phase of one kernel with the ladder it
+// took some 6 of 20.6 ms). A kernel of its own, so that its registers and code
+// are those of this loop alone. 4 blocks of 128 an SM (128 registers): 3 blocks
+// (168, no spills) 1.42 ms, 6 blocks (80) 1.30 ms but 119 against 112 us on the
+// 384x360 grid.
+__global__ void __launch_bounds__(KC_WARM_TPB, KC_WARM_MIN_BLOCKS) k_implicit_warm(DevState s, const __grid_constant__ ImplArgs a, WarmBuf wb, int lanes) {
+  const double dt = s.coef[a.dt_slot];
+  const int lane = threadIdx.x & 31;
+  const long t = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32 * lanes + lane;
+  long ix, iy, iz;
+  if (lane >= lanes || !implicit_cell(s.gr, a, t, ix, iy, iz)) return;
+  const long nc = s.gr.nc, c = cidx(s.gr, ix, iy, iz);
+  double pp[NV];
+  load_cell(s.p, nc, c, pp);
   Geom g;
-  ImplicitPre pre;
-  int done = 0;  // the learned form's pre-solve state took the core's first exit
-  if (act) {
-    load_cell(s.u, nc, c, uu);
-    load_cell(s.p, nc, c, pp);
-    geom_cell<true>(s, ix, iy, iz, g);
-    if (HARVEST)
-      for (int i = 0; i < NV; ++i) pp00[i] = pp[i];
-    if (guessed) {
-      long nd = (long)s.gr.nx * s.gr.ny * s.gr.nz, td = ix + s.gr.nx * (iy + s.gr.ny * iz);
-      double g0[NV];
-      for (int i = 0; i < NV; ++i) g0[i] = x.guess[i * nd + td];
-      done = implicit_prepare_from(uu, pp, g, dt, a.gam, a.rp, a.op, a.ip, g0, pre);
-    } else {
-      implicit_prepare(pp, g, dt, a.gam, a.op, a.ip, pre);
-    }
+  geom_cell(s, ix, iy, iz, g);
+  const lean::Warm w = lean::warm_start(pp, g, dt, a.gam, a.op, a.ip);
+  wb.v[t] = w.uu;
+  wb.v[wb.n + t] = w.ee;
+  wb.v[2 * wb.n + t] = w.ehat;
+  wb.v[3 * wb.n + t] = w.entr;
+  wb.startwith[t] = w.startwith;
+  if (a.ip.lag_opac) {
+    double lag[4];
+    lean::lag_reference(pp, w.ehat, g, a.gam, a.op, lag);
+    for (int k = 0; k < 4; ++k) wb.v[(4 + k) * wb.n + t] = lag[k];
   }
-  __syncthreads();
-  if (!act) return;
+}
+// Adds a warp's solve counts to the step's counters (one address each for the
+// whole grid): folded over the lanes that call it together.
+__device__ __forceinline__ void implicit_count(DevScalars* sc, bool ok, int iters) {
+  const unsigned m = __activemask();
+  const unsigned it = __reduce_add_sync(m, ok ? (unsigned)iters : 0u);
+  const unsigned n = __popc(__ballot_sync(m, ok)), nf = __popc(m) - n;
+  if ((threadIdx.x & 31) == __ffs(m) - 1) {
+    if (it) atomicAdd(&sc->n_iters, (unsigned long long)it);
+    if (n) atomicAdd(&sc->n_solves, (unsigned long long)n);
+    if (nf) atomicAdd(&sc->n_fail, (unsigned long long)nf);
+  }
+}
+// A cell of the implicit solve in shared memory, [warp][value][lane]: every
+// geom() is a fresh set of loads (volatile), so the metric is live only inside
+// the constraints and the residual that read it. What the later rungs alone read
+// (ref()) stays in global memory.
+struct SharedCell {
+  // gcov 10, gcon 16, sqrt(-g), alpha, gttpert, -1/g^tt, 1/sqrt(-g); then uu0 but
+  // its entropy; then the Jacobian: 56 values, 224 KB for 512 threads
+  enum : int { GEO = 31, U0 = GEO, JAC = GEO + lean::U_ENTR, N = JAC + 16 };
+  volatile double* v;  // this lane's slot of its warp's block
+  const double* p_uu;  // the pre-solve u_int, density
+  const double* p_rho;
+  const double* w;  // the warm start: uu, ee, ehat, conserved entropy, lag_opac's four, ws apart
+  long ws;
+  double dt_;
+  int lag;
+  static constexpr size_t bytes(int threads, int extra = 0) { return (size_t)(N + extra) * 8 * threads; }
+  __device__ __forceinline__ SharedCell(double* smem, int extra = 0)
+      : v(smem + (threadIdx.x / 32) * 32 * (N + extra) + threadIdx.x % 32) {}
+  __device__ __forceinline__ void put(const Geom& g, const double uu0[lean::NU0]) {
+    for (int i = 0; i < 4; ++i)
+      for (int j = i; j < 4; ++j) v[32 * sym10(i, j)] = g.gg[i][j];
+    for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 4; ++j) v[32 * (10 + i * 4 + j)] = g.GG[i][j];
+    v[32 * 26] = g.gdet;
+    v[32 * 27] = g.alpha;
+    v[32 * 28] = g.gttpert;
+    v[32 * 29] = -1.0 / g.GG[0][0];
+    v[32 * 30] = 1.0 / g.gdet;
+    for (int i = 0; i < lean::U_ENTR; ++i) v[32 * (U0 + i)] = uu0[i];
+  }
+  __device__ __forceinline__ lean::CellGeom geom() const {
+    lean::CellGeom q;
+    for (int i = 0; i < 4; ++i)
+      for (int j = i; j < 4; ++j) q.g.gg[i][j] = q.g.gg[j][i] = v[32 * sym10(i, j)];
+    for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 4; ++j) q.g.GG[i][j] = v[32 * (10 + i * 4 + j)];
+    q.g.gdet = v[32 * 26];
+    q.g.alpha = v[32 * 27];
+    q.g.gttpert = v[32 * 28];
+    q.ngtt = v[32 * 29];
+    q.gdinv = v[32 * 30];
+    return q;
+  }
+  __device__ __forceinline__ double gcov(int k) const { return v[32 * sym10(k, k)]; }
+  __device__ __forceinline__ double uu0(int i) const {
+    return i == lean::U_ENTR ? w[3 * ws] : v[32 * (U0 + i)];
+  }
+  __device__ __forceinline__ double jac(int i, int j) const { return v[32 * (JAC + i * 4 + j)]; }
+  __device__ __forceinline__ void set_jac(int i, int j, double x) { v[32 * (JAC + i * 4 + j)] = x; }
+  __device__ __forceinline__ double dt() const { return dt_; }
+  __device__ __forceinline__ lean::RefScalars ref() const {
+    lean::RefScalars r;
+    r.ugas = *p_uu;
+    r.rho = *p_rho;
+    r.ehat = w[2 * ws];
+    if (lag)
+      for (int k = 0; k < 4; ++k) r.lag[k] = w[(4 + k) * ws];
+    return r;
+  }
+};
+// The grid's cells as a source of solves: one cell a lane, its warm start in wb.
+struct StepSrc {
+  const DevState& s;
+  const ImplArgs& a;
+  const WarmBuf& wb;
+  long t, c;
+  long ix, iy, iz;
+  bool given;
   ImplicitResult res;
-  if (done) {
-    res = implicit_first_exit_result(pre.startwith);
-  } else {
-    res = implicit_ladder(uu, pp, g, dt, a.gam, a.rp, a.op, a.ip, pre);
-    if (guessed && !res.ok) {  // the seeded ladder failed: the plain solve
-      atomicAdd(x.n_fallback, 1ULL);
-      res = solve_implicit_lab(uu, pp, g, dt, a.gam, a.rp, a.op, a.ip);
+  __device__ __forceinline__ void start(const SharedCell& cell, double q[NV]) {
+    load_cell(s.p, s.gr.nc, c, q);
+    q[UU] = cell.w[0];
+    q[EE] = cell.w[cell.ws];
+  }
+  __device__ __forceinline__ bool take(SharedCell& cell, double q[NV], int& startwith) {
+    if (given) return false;
+    given = true;
+    const long nc = s.gr.nc;
+    {
+      Geom g;
+      load_cell(s.p, nc, c, q);
+      geom_cell<true>(s, ix, iy, iz, g);
+      double uu0[lean::NU0];
+      lean::RefScalars r;
+      lean::reference(q, 0.0, g, a.gam, a.op, a.ip, uu0, r, false);
+      cell.put(g, uu0);
+    }
+    cell.w = wb.v + t;
+    cell.ws = wb.n;
+    cell.p_uu = s.p + UU * nc + c;
+    cell.p_rho = s.p + RHO * nc + c;
+    cell.dt_ = s.coef[a.dt_slot];
+    cell.lag = a.ip.lag_opac;
+    q[UU] = wb.v[t];
+    q[EE] = wb.v[wb.n + t];
+    startwith = wb.startwith[t];
+    return true;
+  }
+  __device__ __forceinline__ void done(const SharedCell& cell, const double q[NV], const ImplicitResult& r) {
+    res = r;
+    s.flags[5 * s.gr.nc + c] = r.ok ? 0 : -1;
+    if (!r.ok) return;
+    double uu[NV];
+    const lean::CellGeom g = cell.geom();
+    p2u(q, uu, g.g, a.gam);
+    store_cell<true>(s.u, s.gr.nc, c, uu);
+    store_cell<true>(s.p, s.gr.nc, c, q);
+  }
+};
+// The rung ladder of every cell from its warm start. NT sets the register
+// budget, an SM holding NT threads (256: 255 registers, 384: 168, 512: 128);
+// `lanes` of each warp's 32 take a cell.
+// Measured on the 192x180x64 wedge, per launch: 5.9 ms with 384 threads, 6.5 with
+// 256 and with 512 (the plain solve in one kernel, warm start included: 20.6 ms).
+// A pass of the 192x180x8 grid executes 298 M warp instructions here and 94 M in
+// the warm start, 847 M before; what is left is dependent FP64 latency (3.3 of
+// 9.4 warp cycles an issue), the trial's spills (1.8) and instruction fetch (1.4).
+// Small blocks, which would fill an SM's slots as warps end, are slower (32 or 64
+// threads: 7.4 to 7.7 ms): warps that start together stay in the same part of the
+// code. A barrier a trip over the whole block gains nothing on top (6.3 ms).
+#ifndef KC_IMPLICIT_TPB
+#define KC_IMPLICIT_TPB 384
+#endif
+template <int NT>
+__global__ void __launch_bounds__(NT, 1) k_implicit(const __grid_constant__ DevState s, DevScalars* sc,
+                                                    const __grid_constant__ ImplArgs a, const __grid_constant__ WarmBuf wb,
+                                                    int lanes) {
+  extern __shared__ __align__(16) double implicit_smem[];
+  const int lane = threadIdx.x & 31;
+  const long t = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32 * lanes + lane;
+  StepSrc src{s, a, wb, t, 0, 0, 0, 0, false, {}};
+  if (lane >= lanes || !implicit_cell(s.gr, a, t, src.ix, src.iy, src.iz)) return;
+  src.c = cidx(s.gr, src.ix, src.iy, src.iz);
+  SharedCell cell(implicit_smem);
+  lean::solve_cells(src, cell, a.gam, a.rp, a.op, a.ip);
+  __syncwarp(__activemask());
+  implicit_count(sc, src.res.ok, src.res.iters);
+}
+// The learned-guess form and the harvest of training pairs: the same ladder from
+// another start. k_implicit_pick takes the warm start's place: a cell whose
+// pre-solve state already passes the core's first exit is finished there, and the
+// others start from whichever of it and the learned state has the smaller rung-0
+// residual.
+enum : int { START_FLUID = 3, START_LEARNED = 4, START_DONE = 8 };  // of WarmBuf::startwith
+constexpr int KC_PICK_TPB = 128;
+__global__ void __launch_bounds__(KC_PICK_TPB, 3) k_implicit_pick(const __grid_constant__ DevState s, DevScalars* sc,
+                                                                  const __grid_constant__ ImplArgs a,
+                                                                  const __grid_constant__ WarmBuf wb, const double* guess,
+                                                                  int lanes) {
+  extern __shared__ __align__(16) double implicit_smem[];
+  const int lane = threadIdx.x & 31;
+  const long t = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32 * lanes + lane;
+  long ix, iy, iz;
+  if (lane >= lanes || !implicit_cell(s.gr, a, t, ix, iy, iz)) return;
+  const long nc = s.gr.nc, c = cidx(s.gr, ix, iy, iz);
+  const long nd = (long)s.gr.nx * s.gr.ny * s.gr.nz, td = ix + s.gr.nx * (iy + s.gr.ny * iz);
+  SharedCell cell(implicit_smem);
+  double pp[NV];
+  load_cell(s.p, nc, c, pp);
+  int fluid;
+  {
+    Geom g;
+    geom_cell(s, ix, iy, iz, g);
+    ImplicitParams ip = a.ip;
+    ip.start_with_bisect = 0;
+    cell.dt_ = s.coef[a.dt_slot];
+    const lean::Warm w = lean::warm_start(pp, g, cell.dt_, a.gam, a.op, ip);
+    fluid = w.startwith;
+    double uu0[lean::NU0];
+    lean::RefScalars r;
+    lean::reference(pp, 0.0, g, a.gam, a.op, a.ip, uu0, r, false);
+    cell.put(g, uu0);
+    wb.v[t] = w.uu;
+    wb.v[wb.n + t] = w.ee;
+    wb.v[2 * wb.n + t] = w.ehat;
+    wb.v[3 * wb.n + t] = w.entr;
+    if (a.ip.lag_opac) {
+      double lag[4];
+      lean::lag_reference(pp, w.ehat, g, a.gam, a.op, lag);
+      for (int k = 0; k < 4; ++k) wb.v[(4 + k) * wb.n + t] = lag[k];
     }
   }
-  if (HARVEST && x.hx && res.ok && res.rung == 0 && (!x.hfilter || presolve_needs_newton(pp00, g, dt, a))) {
-    unsigned long long k = atomicAdd(x.hcount, 1ULL);
-    if ((long)k < x.hcap) {
-      double ehat = -calc_ff_rtt(pp00, g, nullptr);
-      int sw = (ehat < a.ip.threshold * pp00[UU]) ? PRIM_RAD : PRIM_MHD;
-      mlp_features_raw(pp00, dt, g.gdet, g.alpha, sw, x.hx + k * MLP_IN);
-      mlp_targets_raw(pp00, pp, sw, x.ht + k * MLP_OUT);
+  cell.w = wb.v + t;
+  cell.ws = wb.n;
+  cell.p_uu = s.p + UU * nc + c;
+  cell.p_rho = s.p + RHO * nc + c;
+  cell.lag = a.ip.lag_opac;
+  double e0 = 0.0;
+  bool learned = false, done = false;
+  KC_ROLLED
+  for (int k = 0; k < 2 && !done; ++k) {
+    if (k)
+      for (int i = 0; i < NV; ++i) pp[i] = guess[i * nd + td];
+    const double e = lean::start_residual(cell, pp, fluid, a.gam, a.rp, a.op, a.ip);
+    if (k == 0) e0 = e;
+    else learned = e < e0;
+    done = k == 0 && e < a.ip.conv;
+  }
+  wb.startwith[t] = fluid | (learned ? START_LEARNED : 0) | (done ? START_DONE : 0);
+  if (!done) return;
+  pp[ENTR] = s_from_u(pp[RHO], pp[UU], a.gam);
+  double uu[NV];
+  const lean::CellGeom q = cell.geom();
+  p2u(pp, uu, q.g, a.gam);
+  s.flags[5 * nc + c] = 0;
+  store_cell<true>(s.u, nc, c, uu);
+  store_cell<true>(s.p, nc, c, pp);
+  implicit_count(sc, true, 1);
+}
+// a cell's ladder from its picked (seeded) or warm start; the plain solve where the
+// seeded one fails
+template <bool HARVEST>
+struct ExtSrc : StepSrc {
+  const ImplExtra& x;
+  long nd, td;
+  bool seeded, learned;
+  __device__ __forceinline__ void start(const SharedCell& cell, double q[NV]) {
+    if (learned) {
+      for (int i = 0; i < NV; ++i) q[i] = x.guess[i * nd + td];
+      return;
     }
+    StepSrc::start(cell, q);
   }
-  if (res.ok) {
-    store_cell<true>(s.u, nc, c, uu);
-    store_cell<true>(s.p, nc, c, pp);
-    s.flags[5 * nc + c] = 0;
-    atomicAdd(&sc->n_iters, (unsigned long long)res.iters);
-    atomicAdd(&sc->n_solves, 1ULL);
-  } else {
-    s.flags[5 * nc + c] = -1;
-    atomicAdd(&sc->n_fail, 1ULL);
+  __device__ __forceinline__ bool take(SharedCell& cell, double q[NV], int& startwith) {
+    if (!given) {
+      StepSrc::take(cell, q, startwith);
+      startwith &= START_FLUID;
+      if (learned) start(cell, q);
+      return true;
+    }
+    if (res.ok || !seeded) return false;
+    seeded = learned = false;
+    atomicAdd(x.n_fallback, 1ULL);
+    load_cell(s.p, s.gr.nc, c, q);
+    const lean::CellGeom g = cell.geom();
+    const lean::Warm w = lean::warm_start(q, g.g, cell.dt_, a.gam, a.op, a.ip);
+    wb.v[t] = w.uu;
+    wb.v[wb.n + t] = w.ee;
+    StepSrc::start(cell, q);
+    startwith = w.startwith;
+    return true;
   }
+  __device__ __forceinline__ void done(const SharedCell& cell, const double q[NV], const ImplicitResult& r) {
+    if (HARVEST && x.hx && r.ok && r.rung == 0) {
+      double pp00[NV];
+      load_cell(s.p, s.gr.nc, c, pp00);
+      const lean::CellGeom g = cell.geom();
+      if (!x.hfilter || presolve_needs_newton(pp00, g.g, cell.dt_, a)) {
+        unsigned long long k = atomicAdd(x.hcount, 1ULL);
+        if ((long)k < x.hcap) {
+          const int sw = wb.startwith[t] & START_FLUID;
+          mlp_features_raw(pp00, cell.dt_, g.g.gdet, g.g.alpha, sw, x.hx + k * MLP_IN);
+          mlp_targets_raw(pp00, q, sw, x.ht + k * MLP_OUT);
+        }
+      }
+    }
+    StepSrc::done(cell, q, r);
+  }
+};
+template <bool HARVEST>
+__global__ void __launch_bounds__(KC_IMPLICIT_TPB, 1) k_implicit_ext(const __grid_constant__ DevState s, DevScalars* sc,
+                                                                     const __grid_constant__ ImplArgs a,
+                                                                     const __grid_constant__ WarmBuf wb,
+                                                                     const __grid_constant__ ImplExtra x, int lanes) {
+  extern __shared__ __align__(16) double implicit_smem[];
+  const int lane = threadIdx.x & 31;
+  const long t = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32 * lanes + lane;
+  ExtSrc<HARVEST> src{{s, a, wb, t, 0, 0, 0, 0, false, {}}, x, 0, 0, x.guess != nullptr, false};
+  if (lane >= lanes || !implicit_cell(s.gr, a, t, src.ix, src.iy, src.iz)) return;
+  if (wb.startwith[t] & START_DONE) return;
+  src.c = cidx(s.gr, src.ix, src.iy, src.iz);
+  src.nd = (long)s.gr.nx * s.gr.ny * s.gr.nz;
+  src.td = src.ix + s.gr.nx * (src.iy + s.gr.ny * src.iz);
+  src.learned = (wb.startwith[t] & START_LEARNED) != 0;
+  SharedCell cell(implicit_smem);
+  lean::solve_cells(src, cell, a.gam, a.rp, a.op, a.ip);
+  __syncwarp(__activemask());
+  implicit_count(sc, src.res.ok, src.res.iters);
 }
 
 // The split form of the implicit pass, bit-identical to k_implicit. Most cells

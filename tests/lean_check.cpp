@@ -1,0 +1,140 @@
+// Compares the engine's lean implicit solve and W inversion
+// (koral-zig_b200/csrc/kc_implicit_lean.cuh, kc_u2p_lean.cuh) with the plain
+// restatement (include/koral/kimplicit.h, kinvert.h) bit for bit, on the host.
+// Input: cells (geom23, dt, pp), an option variant; prints the number of cells
+// that differ, the number solved and a histogram of the rungs reached.
+#include <cstdint>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <vector>
+
+#include "../include/koral/kparams.h"
+#include "../koral-zig_b200/csrc/kc_implicit_lean.cuh"
+
+using namespace kp;
+
+static void geom_from_record(const double* v, Geom& g) {
+  memset(&g, 0, sizeof g);
+  int n = 0;
+  for (int i = 0; i < 4; ++i)
+    for (int j = i; j < 4; ++j) {
+      g.gg[i][j] = g.gg[j][i] = v[n];
+      g.GG[i][j] = g.GG[j][i] = v[10 + n];
+      ++n;
+    }
+  g.gdet = v[20];
+  g.alpha = v[21];
+  g.gttpert = v[22];
+}
+static bool same(const double* a, const double* b, int n) {
+  for (int i = 0; i < n; ++i)
+    if (memcmp(&a[i], &b[i], 8) != 0 && !(a[i] != a[i] && b[i] != b[i])) return false;
+  return true;
+}
+
+// bases of powers: field values, extremes and special values in turn
+static double k_pow_arg(long c, const double* pp) {
+  const double special[8] = {0.0, 1.0, -2.0, kmath::inf(), kmath::nan(), 1e-300, 3e200, 5e-324};
+  return c % 16 == 0 ? special[(c / 16) % 8] : c % 3 == 0 ? pp[UU] : c % 3 == 1 ? pp[RHO] : pp[EE] * 1e-40;
+}
+int main(int argc, char** argv) {
+  if (argc < 4) return 2;
+  const long n = atol(argv[2]);
+  const int variant = atoi(argv[3]);
+  std::vector<double> in(n * 37);
+  FILE* f = fopen(argv[1], "rb");
+  if (!f || fread(in.data(), 8, in.size(), f) != in.size()) return 3;
+  fclose(f);
+  const double gam = variant == 9 ? 4.0 / 3.0 : 5.0 / 3.0;
+  ImplicitParams ip = implicit_params_puffy();
+  RadParams rp = rad_params_puffy();
+  OpacParams op = opac_params_puffy();
+  if (variant == 1) ip.start_with_bisect = 0;
+  if (variant == 2) ip.scale_jacobian = 0;
+  if (variant == 3) ip.lag_opac = 1;
+  if (variant == 4) ip.allow_rad_ceiling = 0, ip.allow_entr_in_4dprim = 0;
+  if (variant == 5) ip.opdamp_maxlevels = 1, ip.maxiter = 9;
+  if (variant == 6) op.ch.synchrotron_bridge = 1;
+  if (variant == 7) op.ch.comptonization = 0, op.ch.kleinnishina = 0;
+  if (variant == 8) op.ch.synchrotron = 0, op.kappaes_mode = KAPPAES_NONE;
+  if (variant == 10) op.ch.bremsstrahlung = 0, ip.maxiter = 20;
+  if (variant == 11) ip.convrelerr = 1.0e-12, ip.convrel = 1.0e-13;  // many iterations
+  long bad = 0, bad_w = 0, ok = 0, rungs[7] = {0};
+  for (long c = 0; c < n; ++c) {
+    Geom g;
+    geom_from_record(&in[c * 37], g);
+    const double dt = in[c * 37 + 23];
+    double pp[NV], uu[NV], pl[NV], ul[NV];
+    memcpy(pp, &in[c * 37 + 24], sizeof pp);
+    memcpy(pl, pp, sizeof pl);
+    memset(uu, 0, sizeof uu);
+    memset(ul, 0, sizeof ul);
+    const double* pp00 = &in[c * 37 + 24];
+    const ImplicitResult a = solve_implicit_lab(uu, pp, g, dt, gam, rp, op, ip);
+    const kc::lean::Warm w = kc::lean::warm_start(pl, g, dt, gam, op, ip);
+    double uu0[kc::lean::NU0];
+    kc::lean::RefScalars rs;
+    kc::lean::reference(pl, w.ehat, g, gam, op, ip, uu0, rs, true);
+    kc::lean::LocalCell cell;
+    cell.init(g, dt, uu0, rs);
+    struct Src {
+      const double* pp00;
+      const kc::lean::Warm* w;
+      double* out;
+      ImplicitResult res;
+      bool given;
+      void start(const kc::lean::LocalCell&, double q[NV]) {
+        memcpy(q, pp00, sizeof(double) * NV);
+        q[UU] = w->uu;
+        q[EE] = w->ee;
+      }
+      bool take(kc::lean::LocalCell& cell, double q[NV], int& startwith) {
+        if (given) return false;
+        given = true;
+        start(cell, q);
+        startwith = w->startwith;
+        return true;
+      }
+      void done(kc::lean::LocalCell&, double q[NV], const ImplicitResult& r) {
+        res = r;
+        memcpy(out, q, sizeof(double) * NV);
+      }
+    } src = {pp00, &w, pl, {}, false};
+    kc::lean::solve_cells(src, cell, gam, rp, op, ip);
+    const ImplicitResult b = src.res;
+    if (b.ok) p2u(pl, ul, g, gam);
+    else memcpy(pl, pp00, sizeof pl);
+    if (memcmp(&a, &b, sizeof a) != 0 || !same(pp, pl, NV) || !same(uu, ul, NV)) {
+      if (bad < 3) fprintf(stderr, "cell %ld: ok %d/%d rung %d/%d iters %d/%d\n", c, a.ok, b.ok, a.rung, b.rung, a.iters, b.iters);
+      ++bad;
+    }
+    ok += a.ok;
+    rungs[a.rung + 1] += 1;
+    for (double y : {1.5, 1.0 / (gam - 1.0), 1.0 + 1.0 / (gam - 1.0), 0.3, 0.7, 1.0, 2.7, 3.2, 0.5, 2.0}) {
+      const double x = k_pow_arg(c, pp00), r0 = kmath::pow(x, y), r1 = kc::lean::pow_pos(x, y);
+      bad_w += !same(&r0, &r1, 1);
+    }
+    // the W inversion from a displaced guess, hot and entropy, and of broken conserveds
+    p2u(pp00, uu, g, gam);
+    for (int k = 0; k < 4; ++k) {
+      double u2[NV], p1[NV], p2[NV];
+      memcpy(u2, uu, sizeof u2);
+      memcpy(p1, pp00, sizeof p1);
+      const double h = 1.0 + 0.3 * ((double)((c * 7 + k * 13) % 17) / 17.0 - 0.5);
+      p1[RHO] *= h;
+      p1[UU] /= h * h;
+      p1[VX] *= h;
+      if (k == 2) u2[UU] = u2[RHO] * 0.3;
+      if (k == 3) u2[RHO] = -u2[RHO];
+      memcpy(p2, p1, sizeof p2);
+      const int et = k == 1 ? ETYPE_ENTROPY : ETYPE_HOT;
+      const int ra = u2p_solver_w_inl(u2, p1, g, et, gam), rb = kc::lean::u2p_w(u2, p2, g, et, gam, true);
+      if (ra != rb || !same(p1, p2, NV)) ++bad_w;
+    }
+  }
+  printf("%ld %ld %ld", bad, bad_w, ok);
+  for (long x : rungs) printf(" %ld", x);
+  printf("\n");
+  return 0;
+}
