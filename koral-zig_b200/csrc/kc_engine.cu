@@ -311,33 +311,15 @@ void launch_set_bc(kc_handle* h) {
   const DGrid& gr = h->gr;
   BcArgs a = bc_args(h);
   cudaStream_t st = h->stream;
-  if (gr.ngx > 0) {
+  const unsigned bx = nblk(2L * gr.ngx * gr.ny * gr.nz), by = nblk(2L * gr.ngy * gr.nx * gr.nz),
+                 bz = nblk(2L * gr.ngz * gr.nx * gr.ny);
+  ++h->n_launch;
+  k_bc_faces<<<bx + by + bz, TPB, 0, st>>>(h->ds, h->dsc, a, bx, bx + by);
+  if (gr.nx > 1 && gr.ny > 1) {
+    const long ng = gr.ng;
+    const long n = gr.nz == 1 ? 4 * 2 * ng : 4L * ((long)gr.nx + gr.ny + gr.nz) * 2 * ng + 8 * ng * ng * ng;
     ++h->n_launch;
-    k_bc_faces<<<nblk(2L * gr.ngx * gr.ny * gr.nz), TPB, 0, st>>>(h->ds, h->dsc, a, 0);
-  }
-  if (gr.ngy > 0) {
-    ++h->n_launch;
-    k_bc_faces<<<nblk(2L * gr.ngy * gr.nx * gr.nz), TPB, 0, st>>>(h->ds, h->dsc, a, 1);
-  }
-  if (gr.ngz > 0) {
-    ++h->n_launch;
-    k_bc_faces<<<nblk(2L * gr.ngz * gr.nx * gr.ny), TPB, 0, st>>>(h->ds, h->dsc, a, 2);
-  }
-  if (gr.ny > 1 && gr.nz == 1) {
-    ++h->n_launch;
-    k_corners_2d<<<1, 32, 0, st>>>(h->ds, a);
-  } else if (gr.nz > 1 && gr.ny > 1) {
-    long ng = gr.ng;
-    const int planes[3][3] = {{0, 1, 2}, {0, 2, 1}, {1, 2, 0}};
-    long nt0 = 2 * (ng - 1) + 1;
-    for (const auto& pl : planes) {
-      long nslice = (pl[2] == 0 ? gr.nx : pl[2] == 1 ? gr.ny : gr.nz) + 2 * ng;
-      h->n_launch += 2;
-      k_edge_tubes<<<nblk(4L * nslice * nt0, 64), 64, 0, st>>>(h->ds, a.gam, pl[0], pl[1], pl[2], 0);
-      k_edge_tubes<<<nblk(4L * nslice, 64), 64, 0, st>>>(h->ds, a.gam, pl[0], pl[1], pl[2], 1);
-    }
-    ++h->n_launch;
-    k_corner_cubes<<<nblk(8 * ng * ng * ng, 64), 64, 0, st>>>(h->ds, a.gam);
+    k_corners<<<nblk(n, 64), 64, 0, st>>>(h->ds, a);
   }
 }
 

@@ -506,38 +506,37 @@ struct BcArgs {
   int bc[3];
   double gam;
 };
-// ghost faces of one axis; thread t -> (ghost layer i, two transverse indices)
-__global__ void __launch_bounds__(128, KC_BC_MIN_BLOCKS) k_bc_faces(DevState s, DevScalars* sc, BcArgs a, int axis) {
-  long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  long nx = s.gr.nx, ny = s.gr.ny, nz = s.gr.nz;
+// The ghost faces of all axes in one launch: they read domain cells only, so the
+// three axes are independent. Bound by launch latency and one chain of loads and
+// p2u per cell: 8 us on small grids, where three launches took 18. Blocks [0, b1) fill the x faces, [b1, b2) the y
+// faces, the rest the z faces; thread -> (ghost layer i, two transverse indices).
+__global__ void __launch_bounds__(128, KC_BC_MIN_BLOCKS) k_bc_faces(DevState s, DevScalars* sc, BcArgs a, unsigned b1,
+                                                                    unsigned b2) {
+  const int axis = blockIdx.x < b1 ? 0 : blockIdx.x < b2 ? 1 : 2;
+  const long t = (long)(blockIdx.x - (axis == 0 ? 0u : axis == 1 ? b1 : b2)) * blockDim.x + threadIdx.x;
+  const long nx = s.gr.nx, ny = s.gr.ny, nz = s.gr.nz;
   if (axis == 0) {
-    long ng = s.gr.ngx;
-    long n = 2 * ng * ny * nz;
-    if (t >= n) return;
-    long side = t % 2, q = t / 2;
-    long i = 1 + q % ng;
-    q /= ng;
-    long iy = q % ny, iz = q / ny;
+    const long ng = s.gr.ngx;
+    if (t >= 2 * ng * ny * nz) return;
+    const long side = t % 2, q = t / 2;
+    const long i = 1 + q % ng, r = q / ng;
+    const long iy = r % ny, iz = r / ny;
     if (side == 0) bc_cell(s, sc, -i, iy, iz, 0, a.bc, a.gam);
     else bc_cell(s, sc, nx - 1 + i, iy, iz, 1, a.bc, a.gam);
   } else if (axis == 1) {
-    long ng = s.gr.ngy;
-    long n = 2 * ng * nx * nz;
-    if (t >= n) return;
-    long ix = t % nx, q = t / nx;
-    long side = q % 2;
-    q /= 2;
-    long i = 1 + q % ng, iz = q / ng;
+    const long ng = s.gr.ngy;
+    if (t >= 2 * ng * nx * nz) return;
+    const long ix = t % nx, q = t / nx;
+    const long side = q % 2, r = q / 2;
+    const long i = 1 + r % ng, iz = r / ng;
     if (side == 0) bc_cell(s, sc, ix, -i, iz, 2, a.bc, a.gam);
     else bc_cell(s, sc, ix, ny - 1 + i, iz, 3, a.bc, a.gam);
   } else {
-    long ng = s.gr.ngz;
-    long n = 2 * ng * nx * ny;
-    if (t >= n) return;
-    long ix = t % nx, q = t / nx;
-    long iy = q % ny;
-    q /= ny;
-    long side = q % 2, i = 1 + q / 2;
+    const long ng = s.gr.ngz;
+    if (t >= 2 * ng * nx * ny) return;
+    const long ix = t % nx, q = t / nx;
+    const long iy = q % ny, r = q / ny;
+    const long side = r % 2, i = 1 + r / 2;
     if (side == 0) bc_cell(s, sc, ix, iy, -i, 4, a.bc, a.gam);
     else bc_cell(s, sc, ix, iy, nz - 1 + i, 5, a.bc, a.gam);
   }
@@ -565,124 +564,95 @@ __device__ void avg_p_cell(const DevState& s, const long d[3], const long a[3], 
   store_cell(s.p, nc, cd, v);
 }
 
-// 2D corner surfaces + diagonals (bc.zig:256): one thread per corner, the
-// strip -> diagonal order inside a corner kept serial
-__global__ void k_corners_2d(DevState s, BcArgs a) {
-  int corner = threadIdx.x;
-  if (corner >= 4) return;
-  long nx = s.gr.nx, ny = s.gr.ny, ng = s.gr.ng;
-  bool px = a.bc[0] == KC_BC_PERIODIC, py = a.bc[1] == KC_BC_PERIODIC;
-  bool xh = corner & 1, yh = corner & 2;
-  for (long i = 0; i < ng - 1; ++i) {
-    long ax = xh ? nx + i + 1 : -ng + i, ay = yh ? ny : -1, asy = yh ? ny - 1 : 0;
-    copy_p_cell(s, ax, ay, 0, ax, asy, 0);
-    p2u_cell(s, ax, ay, 0, a.gam);
-    long bx = xh ? nx : -1, bsx = xh ? nx - 1 : 0, by = yh ? ny + i + 1 : -ng + i;
-    copy_p_cell(s, bx, by, 0, bsx, by, 0);
-    p2u_cell(s, bx, by, 0, a.gam);
-  }
-  long s1[4], s2[4], d1[3], d2[3];
-  if (!xh && !yh) {
-    long t1[4] = {-1, 0, 0, -1}, t2[4] = {-2, -1, -1, -2};
-    if (py) { t1[0] = -1; t1[1] = ny - 1; t1[2] = -1; t1[3] = ny - 1; t2[0] = -2; t2[1] = ny - 2; t2[2] = -2; t2[3] = ny - 2; }
-    if (px) { t1[0] = nx - 1; t1[1] = -1; t1[2] = nx - 1; t1[3] = -1; t2[0] = nx - 2; t2[1] = -2; t2[2] = nx - 2; t2[3] = -2; }
-    for (int k = 0; k < 4; ++k) { s1[k] = t1[k]; s2[k] = t2[k]; }
-    d1[0] = -1; d1[1] = -1; d2[0] = -2; d2[1] = -2;
-  } else if (!xh && yh) {
-    long t1[4] = {-1, ny - 1, 0, ny}, t2[4] = {-2, ny, -1, ny + 1};
-    if (py) { t1[0] = -1; t1[1] = 0; t1[2] = -1; t1[3] = 0; t2[0] = -2; t2[1] = 1; t2[2] = -2; t2[3] = 1; }
-    if (px) { t1[0] = nx - 1; t1[1] = ny; t1[2] = nx - 1; t1[3] = ny; t2[0] = nx - 2; t2[1] = ny + 1; t2[2] = nx - 2; t2[3] = ny + 1; }
-    for (int k = 0; k < 4; ++k) { s1[k] = t1[k]; s2[k] = t2[k]; }
-    d1[0] = -1; d1[1] = ny; d2[0] = -2; d2[1] = ny + 1;
-  } else if (xh && !yh) {
-    long t1[4] = {nx - 1, -1, nx, 0}, t2[4] = {nx, -2, nx + 1, -1};
-    if (py) { t1[0] = nx; t1[1] = ny - 1; t1[2] = nx; t1[3] = ny - 1; t2[0] = nx + 1; t2[1] = ny - 2; t2[2] = nx + 1; t2[3] = ny - 2; }
-    if (px) { t1[0] = 0; t1[1] = -1; t1[2] = 0; t1[3] = -1; t2[0] = 1; t2[1] = -2; t2[2] = 1; t2[3] = -2; }
-    for (int k = 0; k < 4; ++k) { s1[k] = t1[k]; s2[k] = t2[k]; }
-    d1[0] = nx; d1[1] = -1; d2[0] = nx + 1; d2[1] = -2;
-  } else {
-    long t1[4] = {nx - 1, ny, nx, ny - 1}, t2[4] = {nx, ny + 1, nx + 1, ny};
-    if (py) { t1[0] = nx; t1[1] = 0; t1[2] = nx; t1[3] = 0; t2[0] = nx + 1; t2[1] = 1; t2[2] = nx + 1; t2[3] = 1; }
-    if (px) { t1[0] = 0; t1[1] = ny; t1[2] = 0; t1[3] = ny; t2[0] = 1; t2[1] = ny + 1; t2[2] = 1; t2[3] = ny + 1; }
-    for (int k = 0; k < 4; ++k) { s1[k] = t1[k]; s2[k] = t2[k]; }
-    d1[0] = nx; d1[1] = ny; d2[0] = nx + 1; d2[1] = ny + 1;
-  }
-  d1[2] = 0;
-  d2[2] = 0;
-  long a1[3] = {s1[0], s1[1], 0}, b1[3] = {s1[2], s1[3], 0};
-  avg_p_cell(s, d1, a1, b1);
-  p2u_cell(s, d1[0], d1[1], 0, a.gam);
-  long a2[3] = {s2[0], s2[1], 0}, b2[3] = {s2[2], s2[3], 0};
-  avg_p_cell(s, d2, a2, b2);
-  p2u_cell(s, d2[0], d2[1], 0, a.gam);
-}
-
-// one group of four 3D edge tubes (bc.zig:404): thread -> (tube, slice)
-// The four edge tubes of the (pa, pb) plane along pc (bc.zig:420), in two
-// phases. Phase 0: per (tube, cc), the 2 (ng-1) copies from the face ghosts and
-// the (g1, g1) average, all independent (each writes its own cell and reads
-// face ghosts only), one thread each. Phase 1: the (g2, g2) average, which
-// reads two cells phase 0 wrote. Same values as one thread doing them in order.
+// The corner ghosts, one thread per cell. The reference fills them in groups whose
+// later members read cells that earlier ones wrote; each such cell is a copy of a
+// face ghost, so a thread reads the face ghost itself and all are independent.
+//
+// Around an edge of the (pa, pb) plane (bc.zig:256 in 2D, :404 in 3D) a corner has
+// 2 (ng-1) strip cells, (a outer, b first) and (a first, b outer), copies of the
+// face ghosts beside them, the mean of its two adjoining face ghosts at (first,
+// first), and at (second, second) the mean of two strip cells.
 __device__ __forceinline__ void tube_cell(int pa, int pb, int pc, long av, long bv, long cv, long o[3]) {
   o[pa] = av;
   o[pb] = bv;
   o[pc] = cv;
 }
-__global__ void k_edge_tubes(DevState s, double gam, int pa, int pb, int pc, int phase) {
-  long dims[3] = {s.gr.nx, s.gr.ny, s.gr.nz};
-  long ng = s.gr.ng;
-  long nslice = dims[pc] + 2 * ng;
-  long ntask = phase == 0 ? 2 * (ng - 1) + 1 : 1;
-  long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 4 * nslice * ntask) return;
-  long task = t % ntask, q = t / ntask;
-  int tube = (int)(q / nslice);
-  long cc = -ng + q % nslice;
-  bool a_hi = tube & 2, b_hi = tube & 1;
-  long na = dims[pa], nb = dims[pb];
-  long a_edge = a_hi ? na - 1 : 0, a_g1 = a_hi ? na : -1, a_g2 = a_hi ? na + 1 : -2;
-  long b_edge = b_hi ? nb - 1 : 0, b_g1 = b_hi ? nb : -1, b_g2 = b_hi ? nb + 1 : -2;
+// per_a, per_b: a 2D grid periodic in that direction takes the means' sources
+// from across it (bc.zig:256); a 3D edge never does
+__device__ void corner_edge_cell(const DevState& s, double gam, int pa, int pb, int pc, long cc, int tube, long task,
+                                 bool per_a, bool per_b) {
+  const long dims[3] = {s.gr.nx, s.gr.ny, s.gr.nz};
+  const long ng = s.gr.ng, na = dims[pa], nb = dims[pb];
+  const bool a_hi = tube & 2, b_hi = tube & 1;
+  const long a_edge = a_hi ? na - 1 : 0, b_edge = b_hi ? nb - 1 : 0;
+  const long nstrip = 2 * (ng - 1);
   long d[3], x[3], y[3];
-  if (phase == 1) {
-    tube_cell(pa, pb, pc, a_g2, b_g2, cc, d);
-    tube_cell(pa, pb, pc, a_g2, b_g1, cc, x);
-    tube_cell(pa, pb, pc, a_g1, b_g2, cc, y);
-    avg_p_cell(s, d, x, y);
-  } else if (task == 2 * (ng - 1)) {
-    tube_cell(pa, pb, pc, a_g1, b_g1, cc, d);
-    tube_cell(pa, pb, pc, a_g1, b_edge, cc, x);
-    tube_cell(pa, pb, pc, a_edge, b_g1, cc, y);
-    avg_p_cell(s, d, x, y);
-  } else {
-    long i = task >> 1;
-    long a_out = a_hi ? na + i + 1 : -ng + i;
-    long b_out = b_hi ? nb + i + 1 : -ng + i;
+  if (task < nstrip) {
+    const long i = task >> 1;
     if ((task & 1) == 0) {
-      tube_cell(pa, pb, pc, a_out, b_g1, cc, d);
+      const long a_out = a_hi ? na + i + 1 : -ng + i;
+      tube_cell(pa, pb, pc, a_out, b_hi ? nb : -1, cc, d);
       tube_cell(pa, pb, pc, a_out, b_edge, cc, x);
     } else {
-      tube_cell(pa, pb, pc, a_g1, b_out, cc, d);
+      const long b_out = b_hi ? nb + i + 1 : -ng + i;
+      tube_cell(pa, pb, pc, a_hi ? na : -1, b_out, cc, d);
       tube_cell(pa, pb, pc, a_edge, b_out, cc, x);
     }
     copy_p_cell(s, d[0], d[1], d[2], x[0], x[1], x[2]);
+  } else {
+    const long k = task - nstrip;  // 0: (first, first), 1: (second, second)
+    const long a_g = a_hi ? na + k : -1 - k, b_g = b_hi ? nb + k : -1 - k;
+    tube_cell(pa, pb, pc, a_g, b_g, cc, d);
+    if (per_a) {  // both sources the b ghost across the periodic a
+      tube_cell(pa, pb, pc, a_hi ? k : na - 1 - k, b_g, cc, x);
+      tube_cell(pa, pb, pc, a_hi ? k : na - 1 - k, b_g, cc, y);
+    } else if (per_b) {
+      tube_cell(pa, pb, pc, a_g, b_hi ? k : nb - 1 - k, cc, x);
+      tube_cell(pa, pb, pc, a_g, b_hi ? k : nb - 1 - k, cc, y);
+    } else {
+      // k = 1: the strip cells (a second, b first), (a first, b second) are
+      // copies of these
+      tube_cell(pa, pb, pc, a_g, b_edge, cc, x);
+      tube_cell(pa, pb, pc, a_edge, b_g, cc, y);
+    }
+    avg_p_cell(s, d, x, y);
   }
   p2u_cell(s, d[0], d[1], d[2], gam);
 }
-// the 8 corner cubes (bc.zig:457)
-// Every cube cell copies its cube's domain corner cell, which no cube writes,
-// so the 8 x ng^3 cells are independent: one thread each.
-__global__ void k_corner_cubes(DevState s, double gam) {
-  long ng = s.gr.ng;
-  long per = ng * ng * ng;
+// 2D: the four corners. 3D: the edges along z, y and x over the domain, and the 8
+// corner cubes (bc.zig:457), copies of the domain's corner cells (the reference's
+// edges also run through the cubes, which then overwrite them).
+__global__ void __launch_bounds__(64) k_corners(DevState s, BcArgs a) {
   long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long nx = s.gr.nx, ny = s.gr.ny, nz = s.gr.nz, ng = s.gr.ng;
+  const long ntask = 2 * ng;
+  if (nz == 1) {
+    if (t >= 4 * ntask) return;
+    // corner bit 0: x high, bit 1: y high
+    const int corner = (int)(t / ntask);
+    const int tube = (corner & 1) * 2 + (corner >> 1);
+    const bool px = a.bc[0] == KC_BC_PERIODIC, py = a.bc[1] == KC_BC_PERIODIC;
+    corner_edge_cell(s, a.gam, 0, 1, 2, 0, tube, t % ntask, px, py);
+    return;
+  }
+  for (int e = 0; e < 3; ++e) {
+    const int pa = e == 2 ? 1 : 0, pb = e == 0 ? 1 : 2, pc = 2 - e;
+    const long len = pc == 0 ? nx : pc == 1 ? ny : nz;
+    if (t < 4 * len * ntask) {
+      const long q = t / ntask;
+      corner_edge_cell(s, a.gam, pa, pb, pc, q % len, (int)(q / len), t % ntask, false, false);
+      return;
+    }
+    t -= 4 * len * ntask;
+  }
+  const long per = ng * ng * ng;
   if (t >= 8 * per) return;
-  int cube = (int)(t / per);
+  const int cube = (int)(t / per);
   t %= per;
-  long nx = s.gr.nx, ny = s.gr.ny, nz = s.gr.nz;
-  bool xh = cube & 1, yh = cube & 2, zh = cube & 4;
-  long ix = (xh ? nx : -ng) + t % ng, iy = (yh ? ny : -ng) + (t / ng) % ng, iz = (zh ? nz : -ng) + t / (ng * ng);
+  const bool xh = cube & 1, yh = cube & 2, zh = cube & 4;
+  const long ix = (xh ? nx : -ng) + t % ng, iy = (yh ? ny : -ng) + (t / ng) % ng, iz = (zh ? nz : -ng) + t / (ng * ng);
   copy_p_cell(s, ix, iy, iz, xh ? nx - 1 : 0, yh ? ny - 1 : 0, zh ? nz - 1 : 0);
-  p2u_cell(s, ix, iy, iz, gam);
+  p2u_cell(s, ix, iy, iz, a.gam);
 }
 
 // ---- polar axis overwrite (koral/sim/polaraxis.zig:124) -----------------------
