@@ -17,6 +17,7 @@
 #include <cub/device/device_radix_sort.cuh>
 
 #include "kc_kernels.cuh"
+#include "kc_init_lean.cuh"
 #include "../../include/koral/kdump.h"
 #include "../../include/koral/kinit.h"
 
@@ -26,6 +27,7 @@ using namespace kc;
 namespace {
 
 const int TPB = 128;
+const int INIT_TPB = 64;  // of the column kernel: two warps a block
 inline unsigned nblk(long n, int tpb = TPB) { return (unsigned)((n + tpb - 1) / tpb); }
 
 template <class Fn>
@@ -804,22 +806,28 @@ int run_step(kc_handle* h, double forced_dt, kc_step_info* info) {
   return st;
 }
 
-// The limotorus profile of (x1, x2) columns [c0, c0 + n) (tools.c
+// The limotorus profile of the (x1, x2) columns (tools.c
 // init_dsandvels_limotorus, puffy.zig:572: angular-momentum root finding and
-// the adaptive GK21 quadrature of ln f), one thread per column; each thread's
-// quadrature segment table is its slice of `seg` (4 kMaxSeg doubles).
-__global__ void __launch_bounds__(128) k_init_columns(Grid g, MetricParams mp, kcinit::TorusConsts tc,
-                                                      kcinit::PuffyPhysics ph, long c0, long n, double* dvcol,
-                                                      double* seg) {
-  long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  long col = c0 + k, ix = col % g.nx, iy = col / g.nx;
-  Geom gb0;
-  geometry_bl_at(g, mp, ix, iy, 0, gb0);
-  kcinit::DsVels dv = kcinit::init_dsandvels_s(gb0.xx[1], gb0.xx[2], mp.a, tc, ph, seg + k * 4L * kcinit::kMaxSeg);
-  dvcol[3 * col] = dv.rho;
-  dvcol[3 * col + 1] = dv.uu;
-  dvcol[3 * col + 2] = dv.ell;
+// the adaptive GK21 quadrature of ln f), one warp per column (kc_init_lean.cuh);
+// each warp's quadrature segment table is its slice of `seg` (4 kMaxSeg doubles).
+__global__ void __launch_bounds__(INIT_TPB) k_init_columns(Grid g, MetricParams mp, kcinit::TorusConsts tc,
+                                                           kcinit::PuffyPhysics ph, long ncol, double* dvcol,
+                                                           double* seg) {
+  const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32, nwarp = (long)gridDim.x * blockDim.x / 32;
+  const lean::TorusL t = lean::torus_l(mp.a, tc.lb1, tc.lb2, ph.lt_xi);
+  for (long col = warp; col < ncol; col += nwarp) {
+    const long ix = col % g.nx, iy = col / g.nx;
+    Geom gb0;
+    geometry_bl_at(g, mp, ix, iy, 0, gb0);
+    const kcinit::DsVels dv =
+        lean::init_column_warp(gb0.xx[1], gb0.xx[2], t, tc, ph, seg + warp * 4L * kcinit::kMaxSeg);
+    if (threadIdx.x % 32 == 0) {
+      dvcol[3 * col] = dv.rho;
+      dvcol[3 * col + 1] = dv.uu;
+      dvcol[3 * col + 2] = dv.ell;
+    }
+    __syncwarp();
+  }
 }
 
 // PUFFY per-cell initial state (puffy.zig:715 prepInitCellWith, then the
@@ -1475,21 +1483,19 @@ int kc_init_puffy(kc_handle* h, double perturb, double perturb_rho, uint64_t see
   h->last_status = 0;
   h->err.clear();
   // the torus profile per (x1, x2) column (the metric is axisymmetric, so one
-  // solve serves a column), in chunks whose quadrature scratch stays <= 1 GiB
+  // solve serves a column)
   long ncol = (long)g.nx * g.ny;
   int st = 0;
   if (!h->init_dv) h->init_dv = dalloc<double>(h, (size_t)3 * ncol, st);
   if (st) return st;
   double* ddv = h->init_dv;
-  const long chunk = 65536;
-  long nseg = ncol < chunk ? ncol : chunk;
+  // as many warps as the device holds: 16 KB of scratch each
+  const long blocks = 16L * h->nsm, need = (ncol + INIT_TPB / 32 - 1) / (INIT_TPB / 32);
+  const unsigned nb = (unsigned)(need < blocks ? need : blocks);
   DevBufE seg;
-  if (cudaMalloc(&seg.p, (size_t)nseg * 4 * kcinit::kMaxSeg * 8) != cudaSuccess)
+  if (cudaMalloc(&seg.p, (size_t)nb * (INIT_TPB / 32) * 4 * kcinit::kMaxSeg * 8) != cudaSuccess)
     return fail(h, KC_ERR_OOM, "init quadrature scratch");
-  for (long c0 = 0; c0 < ncol; c0 += chunk) {
-    long n = ncol - c0 < chunk ? ncol - c0 : chunk;
-    k_init_columns<<<nblk(n), TPB, 0, h->stream>>>(g, mp, tc, ph, c0, n, ddv, (double*)seg.p);
-  }
+  k_init_columns<<<nb, INIT_TPB, 0, h->stream>>>(g, mp, tc, ph, ncol, ddv, (double*)seg.p);
   st = cuda_check(h, cudaMemsetAsync(h->ds.flags, 0, 6L * nc * sizeof(int), h->stream), "init");
   if (!st) st = cuda_check(h, cudaMemsetAsync(h->ds.vecpot, 0, 6L * nc * sizeof(double), h->stream), "init");
   if (!st) st = cuda_check(h, cudaMemsetAsync(h->ds.p, 0, (size_t)NV * nc * 8, h->stream), "init");

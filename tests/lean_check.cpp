@@ -11,6 +11,7 @@
 
 #include "../include/koral/kparams.h"
 #include "../koral-zig_b200/csrc/kc_implicit_lean.cuh"
+#include "../koral-zig_b200/csrc/kc_init_lean.cuh"
 
 using namespace kp;
 
@@ -38,7 +39,47 @@ static double k_pow_arg(long c, const double* pp) {
   const double special[8] = {0.0, 1.0, -2.0, kmath::inf(), kmath::nan(), 1e-300, 3e200, 5e-324};
   return c % 16 == 0 ? special[(c / 16) % 8] : c % 3 == 0 ? pp[UU] : c % 3 == 1 ? pp[RHO] : pp[EE] * 1e-40;
 }
+// The torus functions of the column solve, and the outer bisection by outcome
+// trees (its walk as the warp makes it), against the serial code
+static int check_init(double a) {
+  kcinit::PuffyPhysics ph;
+  const kcinit::TorusConsts tc = kcinit::torus_consts(a, ph);
+  const kc::lean::TorusL t = kc::lean::torus_l(a, tc.lb1, tc.lb2, ph.lt_xi);
+  const kcinit::LnfIntegrand integrand = {a, tc.lb1, tc.lb2, ph.lt_xi};
+  long bad = 0, n = 0;
+  for (double r = 35.0; r < 499.0; r *= 1.013, ++n) {
+    const double th = 0.4 + 1.1 * (double)(n % 23) / 23.0;
+    const kcinit::Gd gd = kcinit::compute_gd(r, th, a);
+    const double l0 = kcinit::lam_bl(r, gd, a, tc.lb1, tc.lb2, ph.lt_xi), l1 = t.lam_bl(r, gd);
+    const double f0 = integrand(r), f1 = t.lnf(r);
+    bad += !same(&l0, &l1, 1) + !same(&f0, &f1, 1);
+    if (n % 29) continue;
+    const double m0 = kcinit::find_rml(l0, a, tc.lb1, tc.lb2, ph.lt_xi);
+    const double lamsq = l0 * l0, x1 = 6.0, x2 = 10.0 * lamsq;
+    double dx, rtb, m1 = 0.0;
+    if (t.rml_at(x1, lamsq) < 0.0) dx = x2 - x1, rtb = x1;
+    else dx = x1 - x2, rtb = x2;
+    bool found = false;
+    for (int j = 0; j < 100 && !found; j += 5) {
+      const double rtb0 = rtb, dx0 = dx;
+      for (int node = 1; node < 32 && !found;) {
+        dx *= 0.5;
+        const double xmid = rtb + dx, xt = kc::lean::tree_midpoint(node, rtb0, dx0);
+        bad += !same(&xmid, &xt, 1);
+        const double fmid = t.rml_at(xt, lamsq);
+        if (fmid <= 0.0) rtb = xmid;
+        if (kmath::fabs(dx) < kcinit::kXacc || fmid == 0.0) found = true, m1 = rtb;
+        node = 2 * node + (fmid <= 0.0);
+      }
+    }
+    bad += !same(&m0, &m1, 1);
+  }
+  printf("%ld %ld\n", bad, n);
+  return 0;
+}
+
 int main(int argc, char** argv) {
+  if (argc == 3 && !strcmp(argv[1], "init")) return check_init(atof(argv[2]));
   if (argc < 4) return 2;
   const long n = atol(argv[2]);
   const int variant = atoi(argv[3]);

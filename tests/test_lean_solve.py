@@ -1,5 +1,6 @@
-"""The engine's lean implicit solve and W inversion
-(koral-zig_b200/csrc/kc_implicit_lean.cuh, kc_u2p_lean.cuh) against the plain restatement of the reference (include/koral), bit for bit, on
+"""The engine's lean implicit solve, W inversion and torus functions
+(koral-zig_b200/csrc/kc_implicit_lean.cuh, kc_u2p_lean.cuh, kc_init_lean.cuh)
+against the plain restatement of the reference (include/koral), bit for bit, on
 the host: the same source as the kernels, compiled by g++ with lean_check.cpp."""
 import os
 import subprocess
@@ -59,3 +60,9 @@ def test_lean_solve_is_bitwise_the_plain_solve(checker, cells, variant):
     assert bad == 0 and bad_w == 0, r.stderr
     assert ok > 0 and failed > 0 and ok + failed == n and sum(1 for x in rungs if x) >= 3
 
+
+@pytest.mark.parametrize("spin", [0.0, 0.5, -0.3, 0.95])
+def test_torus_functions_are_bitwise_the_plain_ones(checker, spin):
+    r = subprocess.run([checker, "init", str(spin)], check=True, capture_output=True, text=True)
+    bad, n = (int(x) for x in r.stdout.split())
+    assert bad == 0 and n > 100
