@@ -512,7 +512,7 @@ void launch_face_fluxes(kc_handle* h) {
     long n = (dims[dim] + 1) * n0 * n1;
     ++h->n_launch;
     int tb = h->tpb_flux;
-    unsigned nb = nblk(2 * n, tb);  // two lanes a face
+    unsigned nb = nblk(n, tb);
     bool mx = (a.fp32 & (KC_FP32_PPM | KC_FP32_LAXF | KC_FP32_FLUX)) != 0;
     if (dim == 0) {
       if (mx) k_face_flux<true, 0><<<nb, tb, 0, h->stream>>>(h->ds, h->dsc, a);

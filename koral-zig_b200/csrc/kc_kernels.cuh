@@ -794,9 +794,11 @@ __device__ __forceinline__ void face_rijvisc(const DevState& s, long c, long cm,
 // one face state: floors, one-sided flux, viscous addition, conserveds; the
 // floors and the flux inlined (their out-of-line forms passed the state and the
 // face metric through the call frame: 1.17 KB per thread, 27% slower)
-__device__ __forceinline__ int face_state(const DevState& s, const FluxArgs& a, int dim, double pp[NV], const Geom& g,
-                                          long c, long cm, double ff[NV], double uu[NV], int& gc) {
+__device__ int face_state(const DevState& s, DevScalars* sc, const FluxArgs& a, int dim, double pp[NV], const Geom& g,
+                          long c, long cm, double ff[NV], double uu[NV]) {
+  int gc = 0;
   check_floors_mhd_inl(pp, g, a.gam, a.fl, gc);
+  if (gc) atomicAdd(&sc->n_guard, (unsigned long long)gc);
   int e = f_flux_prime_inl(pp, dim, g, a.gam, ff);
   if (e) return e;
   if (a.fp32 & KC_FP32_FLUX)
@@ -819,77 +821,81 @@ __device__ __forceinline__ int face_state(const DevState& s, const FluxArgs& a, 
 // LAXF dissipation, rounded fluxes; kc_mixed.cuh) FluxArgs::fp32 selects
 // DIM: the face direction, a template argument so that every index along it
 // is a compile-time one (one instance per direction)
-// Two lanes a face, one per side: each reconstructs its side's state and forms
-// that state's floors, flux and conserveds, and the pair exchanges them for the
-// LAXF flux. One thread doing both sides holds two states through the code of
-// both and spills (128 registers, 400 bytes); a side alone fits.
 template <bool MIXED, int DIM>
 __global__ void __launch_bounds__(128, KC_FLUX_MIN_BLOCKS) k_face_flux(DevState s, DevScalars* sc, const __grid_constant__ FluxArgs a) {
   constexpr int dim = DIM;
-  constexpr int c0d = dim == 0 ? 1 : 0, c1d = dim == 2 ? 1 : 2;
-  const long dims[3] = {s.gr.nx, s.gr.ny, s.gr.nz};
-  const long n = dims[dim];
-  const long lo0 = dims[c0d] > 1 ? -1 : 0, n0 = dims[c0d] > 1 ? dims[c0d] + 2 : dims[c0d];
-  const long lo1 = dims[c1d] > 1 ? -1 : 0, n1 = dims[c1d] > 1 ? dims[c1d] + 2 : dims[c1d];
-  // the face index walks x fastest: for dim 0 that is the face's own index
-  const long nf0 = dim == 0 ? n + 1 : n0;
-  const long nfo = dim == 0 ? n0 : n + 1;
-  const long tt = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int side = (int)(tt & 1);
-  const long nface = nf0 * nfo * n1;
-  const bool act = (tt >> 1) < nface;
-  const long t = act ? tt >> 1 : nface - 1;  // the idle lanes of the last warp repeat the last face
-  const long a0 = t % nf0, q = t / nf0;
-  const long a1 = q % nfo, a2 = q / nfo;
+  long n = dim == 0 ? s.gr.nx : dim == 1 ? s.gr.ny : s.gr.nz;
+  int c0d = dim == 0 ? 1 : 0, c1d = dim == 2 ? 1 : 2;
+  long dims[3] = {s.gr.nx, s.gr.ny, s.gr.nz};
+  long lo0 = dims[c0d] > 1 ? -1 : 0, n0 = dims[c0d] > 1 ? dims[c0d] + 2 : dims[c0d];
+  long lo1 = dims[c1d] > 1 ? -1 : 0, n1 = dims[c1d] > 1 ? dims[c1d] + 2 : dims[c1d];
+  // thread x walks the x index: for dim 0 that is the face index
+  long nf0 = dim == 0 ? n + 1 : n0;
+  long nfo = dim == 0 ? n0 : n + 1;
+  long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nf0 * nfo * n1) return;
+  long a0 = t % nf0, q = t / nf0;
+  long a1 = q % nfo, a2 = q / nfo;
+  long f, cx0, cx1;
+  if (dim == 0) {
+    f = a0;
+    cx0 = lo0 + a1;
+  } else {
+    cx0 = lo0 + a0;
+    f = a1;
+  }
+  cx1 = lo1 + a2;
   long cf[3];
-  cf[dim] = dim == 0 ? a0 : a1;
-  cf[c0d] = lo0 + (dim == 0 ? a1 : a0);
-  cf[c1d] = lo1 + a2;
-  const long f = cf[dim];
+  cf[dim] = f;
+  cf[c0d] = cx0;
+  cf[c1d] = cx1;
   const Grid& g = s.gr.g;
-  const long nc = s.gr.nc;
-  const long step = dim == 0 ? 1 : dim == 1 ? s.gr.sx : s.gr.sx * s.gr.sy;
-  const long c = cidx(s.gr, cf[0], cf[1], cf[2]), cm = c - step;  // the cells f and f-1
-  double pp[NV];
-  {
-    // this side's cell is f-1+side; its stencil the two cells on either side of it
-    const long c0 = c + (side - 3) * step;
-    double dxs[5];
-    for (int k = 0; k < 5; ++k) dxs[k] = cell_size(g, f - 3 + side + k, dim);
-    PpmCoef kf;  // the width factors of the stencil, shared by the 13 variables
-    if (!MIXED || !(a.fp32 & KC_FP32_PPM)) kf = ppm_coef(dxs);
-    for (int iv = 0; iv < NV; ++iv) {
-      double v[5];
-      for (int k = 0; k < 5; ++k) v[k] = s.p[iv * nc + c0 + k * step];
-      const Faces r = (MIXED && (a.fp32 & KC_FP32_PPM)) ? recon_ppm_mixed(v, dxs) : ppm_apply(v, kf);
-      pp[iv] = side ? r.left : r.right;  // the face is the right one of cell f-1, the left one of cell f
+  long nc = s.gr.nc;
+  // stencil cells f-3 .. f+2 along dim
+  long cst[6];
+  for (int k = 0; k < 6; ++k) {
+    long cc[3] = {cf[0], cf[1], cf[2]};
+    cc[dim] = f - 3 + k;
+    cst[k] = cidx(s.gr, cc[0], cc[1], cc[2]);
+  }
+  double dxs[6];
+  for (int k = 0; k < 6; ++k) dxs[k] = cell_size(g, f - 3 + k, dim);
+  double pL[NV], pR[NV];
+  PpmCoef kl, kr;  // the width factors of the two stencils, shared by the 13 variables
+  if (!MIXED || !(a.fp32 & KC_FP32_PPM)) {
+    kl = ppm_coef(dxs);
+    kr = ppm_coef(dxs + 1);
+  }
+  for (int iv = 0; iv < NV; ++iv) {
+    double v[6];
+    for (int k = 0; k < 6; ++k) v[k] = s.p[iv * nc + cst[k]];
+    if (MIXED && (a.fp32 & KC_FP32_PPM)) {
+      pL[iv] = recon_ppm_mixed(v, dxs).right;
+      pR[iv] = recon_ppm_mixed(v + 1, dxs + 1).left;
+    } else {
+      pL[iv] = ppm_apply(v, kl).right;      // cell f-1: right face value
+      pR[iv] = ppm_apply(v + 1, kr).left;   // cell f: left face value
     }
   }
   Geom geo;
   geom_face(s, cf[0], cf[1], cf[2], dim, geo);
-  double ff[NV], uu[NV];
-  int gc = 0;
-  const int e = face_state(s, a, dim, pp, geo, c, cm, ff, uu, gc);
-  // the left state's error is reported first, and the right state is not looked at then
-  const int e0 = __shfl_sync(0xffffffffu, e, (threadIdx.x & 31) & ~1), e1 = __shfl_sync(0xffffffffu, e, (threadIdx.x & 31) | 1);
-  if (act && gc && (side == 0 || !e0)) atomicAdd(&sc->n_guard, (unsigned long long)gc);
-  if (act && (side == 0 ? e0 : (e0 ? 0 : e1))) set_err(sc, e, c);
-  const double ag = kmath::fmax(s.amax[(long)dim * nc + c], s.amax[(long)dim * nc + cm]);
-  const double agr = kmath::fmax(s.amax[(long)(3 + dim) * nc + c], s.amax[(long)(3 + dim) * nc + cm]);
-  const long fi = face_index(s.gr, dim, cf[0], cf[1], cf[2]);
-  double* out = s.flb[dim];
-  const long nfd = s.nf[dim];
-  const bool store = act && !e0 && !e1;
-#pragma unroll
-  for (int iv = 0; iv < NV; ++iv) {
-    const double fo = __shfl_xor_sync(0xffffffffu, ff[iv], 1), uo = __shfl_xor_sync(0xffffffffu, uu[iv], 1);
-    // the even variables by the left lane, the odd ones by the right
-    if (store && side == (iv & 1)) {
-      const double fl = side ? fo : ff[iv], fr = side ? ff[iv] : fo, ul = side ? uo : uu[iv], ur = side ? uu[iv] : uo;
-      const double l = iv >= EE ? agr : ag;
-      out[iv * nfd + fi] = (MIXED && (a.fp32 & KC_FP32_LAXF)) ? laxf_f(fl, fr, ul, ur, l) : laxf(fl, fr, ul, ur, l);
-    }
+  long c = cst[3], cm = cst[2];
+  double ffl[NV], ffr[NV], uL[NV], uR[NV];
+  int e = face_state(s, sc, a, dim, pL, geo, c, cm, ffl, uL);
+  if (!e) e = face_state(s, sc, a, dim, pR, geo, c, cm, ffr, uR);
+  if (e) {
+    set_err(sc, e, c);
+    return;
   }
+  double ag = kmath::fmax(s.amax[(long)dim * nc + c], s.amax[(long)dim * nc + cm]);
+  double agr = kmath::fmax(s.amax[(long)(3 + dim) * nc + c], s.amax[(long)(3 + dim) * nc + cm]);
+  long fi = face_index(s.gr, dim, cf[0], cf[1], cf[2]);
+  double* out = s.flb[dim];
+  long nfd = s.nf[dim];
+#pragma unroll
+  for (int iv = 0; iv < NV; ++iv)
+    out[iv * nfd + fi] = (MIXED && (a.fp32 & KC_FP32_LAXF)) ? laxf_f(ffl[iv], ffr[iv], uL[iv], uR[iv], iv >= EE ? agr : ag)
+                                                         : laxf(ffl[iv], ffr[iv], uL[iv], uR[iv], iv >= EE ? agr : ag);
 }
 
 // ---- face fluxes through shared-memory tiles (sweeps along y and z) ---------------
@@ -991,10 +997,8 @@ __global__ void __launch_bounds__(128, KC_FLUX_MIN_BLOCKS) k_face_flux_tiled(Dev
   Geom geo;
   geom_face(s, cf[0], cf[1], cf[2], dim, geo);
   double ffl[NV], ffr[NV], uL[NV], uR[NV];
-  int gc = 0;
-  int e = face_state(s, a, dim, pL, geo, c, cm, ffl, uL, gc);
-  if (!e) e = face_state(s, a, dim, pR, geo, c, cm, ffr, uR, gc);
-  if (gc) atomicAdd(&sc->n_guard, (unsigned long long)gc);
+  int e = face_state(s, sc, a, dim, pL, geo, c, cm, ffl, uL);
+  if (!e) e = face_state(s, sc, a, dim, pR, geo, c, cm, ffr, uR);
   if (e) {
     set_err(sc, e, c);
     return;
