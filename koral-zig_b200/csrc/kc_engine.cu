@@ -17,6 +17,7 @@
 #include <cub/device/device_radix_sort.cuh>
 
 #include "kc_kernels.cuh"
+#include "kc_fold.cuh"
 #include "kc_init_lean.cuh"
 #include "../../include/koral/kdump.h"
 #include "../../include/koral/kinit.h"
@@ -1160,10 +1161,22 @@ int kc_scalars(kc_handle* h, double dt, double r_lum, double r_scale, kc_scalar_
   k_diag_mdot<<<nblk(nyz), TPB, 0, h->stream>>>(h->ds, h->dsc, ix_h, dzfac, mdot_t);
   k_diag_lum<<<nblk(nyz), TPB, 0, h->stream>>>(h->ds, h->dsc, ix_l, h->sp.gam, h->lum_gbl, h->lum_w,
                                                  h->lum_w + nyz, rad_t, tot_t);
-  k_fold_ordered<<<1, 256, 0, h->stream>>>(mass_t, ndom, res + 0);
-  k_fold_ordered<<<1, 256, 0, h->stream>>>(mdot_t, nyz, res + 1);
-  k_fold_ordered<<<1, 256, 0, h->stream>>>(rad_t, nyz, res + 2);
-  k_fold_ordered<<<1, 256, 0, h->stream>>>(tot_t, nyz, res + 3);
+  // the four sums in the reference's order (kc_fold.cuh); scratch behind the terms
+  FoldJobs J = {{mass_t, mdot_t, rad_t, tot_t}, {res, res + 1, res + 2, res + 3}, {ndom, nyz, nyz, nyz}, {}};
+  long nch = 0;
+  for (int k = 0; k < FOLD_JOBS; ++k) {
+    J.chunk0[k] = nch;
+    nch += fold_chunks(J.n[k]);
+  }
+  double* sums = scaleth + gr.nx;
+  FoldChunk* chunks = (FoldChunk*)(sums + nch);
+  const int serial = ndom <= FOLD_SERIAL;
+  if (!serial) {
+    const dim3 grid((unsigned)fold_chunks(ndom), FOLD_JOBS);
+    k_fold_sums<<<grid, FOLD_TPB, 0, h->stream>>>(J, sums);
+    k_fold_exact<<<grid, FOLD_TPB, 0, h->stream>>>(J, sums, chunks);
+  }
+  k_fold_finish<<<FOLD_JOBS, 32, 0, h->stream>>>(J, chunks, serial);
   // scale height: the dynamo's per-radius fold (dynamo.zig:239), into a scratch row
   DevState ds2 = h->ds;
   ds2.scaleth = scaleth;

@@ -2010,7 +2010,7 @@ __global__ void __launch_bounds__(128) k_init_beta_scale(DevState s, double gam,
 
 // ---- scalar diagnostics (koral/io/scalars.zig, koral/io/dump.zig:358) ---------
 // Each reduction writes its per-cell terms in the reference's serial loop order
-// and k_fold_ordered adds them in that order, so the sums are the serial ones.
+// and kc_fold.cuh's kernels give the sums in that order.
 
 // per domain cell: the totalMass term (scalars.zig:78) at index
 // ix + nx (iy + ny iz), and the collectDiag counts (non-finite cells, hd flags)
@@ -2090,21 +2090,6 @@ __global__ void __launch_bounds__(128) k_diag_lum(DevState s, DevScalars* sc, lo
   if (rrt < 0.0) rrt = 0.0;
   rad_terms[t] = gb.gdet * rrt * dth[t] * dph[t];
   tot_terms[t] = gb.gdet * (rhour + trt + rrt) * dth[t] * dph[t];
-}
-// out[0] = ((0 + v[0]) + v[1]) + ... in index order: a block stages tiles in
-// shared memory, thread 0 adds them in order
-__global__ void __launch_bounds__(256) k_fold_ordered(const double* v, long n, double* out) {
-  __shared__ double tile[2048];
-  double acc = 0.0;
-  for (long k0 = 0; k0 < n; k0 += 2048) {
-    long m = n - k0 < 2048 ? n - k0 : 2048;
-    for (long k = threadIdx.x; k < m; k += blockDim.x) tile[k] = v[k0 + k];
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (long k = 0; k < m; ++k) acc += tile[k];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *out = acc;
 }
 
 }  // namespace kc

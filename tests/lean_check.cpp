@@ -7,9 +7,11 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <random>
 #include <vector>
 
 #include "../include/koral/kparams.h"
+#include "../koral-zig_b200/csrc/kc_fold.cuh"
 #include "../koral-zig_b200/csrc/kc_implicit_lean.cuh"
 #include "../koral-zig_b200/csrc/kc_init_lean.cuh"
 
@@ -78,7 +80,54 @@ static int check_init(double a) {
   return 0;
 }
 
+// The ordered fold's maps, chunk by chunk, against the serial sum: sums that grow
+// through binades, of one sign and of both, ties (few-bit terms), zeros, a
+// non-finite term
+static int check_fold() {
+  using namespace kc;
+  std::mt19937_64 r(3);
+  long bad = 0, mapped = 0;
+  for (int t = 0; t < 400; ++t) {
+    const int kind = t % 8, chunk = 1 << (5 + t % 4);
+    std::vector<double> v(2000 + r() % 20000);
+    for (double& x : v) {
+      const double u = (double)(r() >> 11) * 0x1p-53;
+      x = kind == 0 ? u : kind == 1 ? ldexp(u, (int)(r() % 60)) : kind == 2 ? -ldexp(u, (int)(r() % 10))
+          : kind == 3 ? (double)(long)(u * 1000) * 0.125 : kind == 4 ? u - 0.3 : kind == 5 ? (r() % 3 ? 0.0 : u * 1e-20)
+          : kind == 6 ? ldexp((double)(1 + r() % 7), -3 + (int)(r() % 4)) : u * 1e-30 * (u < 0.001 ? 1e10 : 1.0);
+    }
+    if (kind == 6) v[0] = ldexp(1.0, 51 + t % 4);
+    if (t % 50 == 49) v[v.size() / 2] = kmath::inf();
+    double s = 0.0, acc = 0.0, est = 0.0;
+    for (double x : v) s += x;
+    for (size_t k0 = 0; k0 < v.size(); k0 += chunk) {
+      const size_t k1 = k0 + chunk < v.size() ? k0 + chunk : v.size();
+      FoldChunk c = {{0, 0}, 0, 0, 0};
+      double sum = 0.0;
+      if (const long long key = fold_key(est * (1.0 + 1e-14))) {
+        std::vector<FoldRun> q;
+        for (size_t k = k0; k < k1; ++k) q.push_back(fold_term(v[k] * fold_scale(key)));
+        while (q.size() > 1) {  // joined as a tree, as the kernel does
+          std::vector<FoldRun> z;
+          for (size_t i = 0; i < q.size(); i += 2) z.push_back(i + 1 < q.size() ? fold_join(q[i], q[i + 1]) : q[i]);
+          q = z;
+        }
+        c = {q[0].m, q[0].lo, q[0].hi, q[0].ok ? key : 0};
+      }
+      if (fold_apply(acc, c)) ++mapped;
+      else
+        for (size_t k = k0; k < k1; ++k) acc += v[k];
+      for (size_t k = k0; k < k1; ++k) sum += v[k];
+      est += sum;
+    }
+    bad += !same(&s, &acc, 1);
+  }
+  printf("%ld %ld\n", bad, mapped);
+  return 0;
+}
+
 int main(int argc, char** argv) {
+  if (argc == 2 && !strcmp(argv[1], "fold")) return check_fold();
   if (argc == 3 && !strcmp(argv[1], "init")) return check_init(atof(argv[2]));
   if (argc < 4) return 2;
   const long n = atol(argv[2]);

@@ -1,0 +1,96 @@
+"""The kernels that replaced plain ones, at the sizes where their own rules change:
+the implicit and u2p passes around the warp's cell counts, the init's columns with
+spin, the ordered folds around the chunk size, the ghost fill on every kind of
+boundary; all bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+from tests.engine import koralcuda
+from tests.orcsim import OracleSim
+
+pytestmark = pytest.mark.gpu
+
+
+def _bits(a):
+    return np.ascontiguousarray(a, dtype=np.float64).view(np.uint64)
+
+
+def _pair(nx, ny, nz, **opt):
+    kc = koralcuda()
+    kc.lib()
+    grid, o = kc.puffy_grid(nx, ny, nz), kc.puffy_options(**opt)
+    gpu, orc = kc.Sim(grid, o), OracleSim(grid, o, nthreads=8)
+    assert gpu.initPuffy(1e-3, 1e-3, 5) == orc.init_puffy(1e-3, 1e-3, 5)
+    orc.lib.orc_sim_init_timestep_guess(orc.h)
+    return gpu, orc
+
+
+def _same(gpu, orc):
+    assert np.array_equal(_bits(gpu.p), _bits(orc.prims()))
+    assert np.array_equal(_bits(gpu.u), _bits(orc.cons()))
+    assert np.array_equal(gpu.flags, orc.flags())
+
+
+@pytest.mark.parametrize("spin", [0.0, 0.5])
+def test_init_columns_with_spin(spin):
+    """The column solve with its angular momentum's powers multiplied away
+    (no spin) and formed (spin); 43 x 37 columns are no multiple of a block's."""
+    gpu, orc = _pair(43, 37, 1, bhspin=spin)
+    _same(gpu, orc)
+
+
+@pytest.mark.parametrize("shape", [(31, 21, 1), (37, 33, 1), (148, 9, 1), (149, 33, 4)])
+def test_steps_at_the_edges_of_the_solve_launches(shape):
+    """651 and 1221 cells (2 and 3 cells a warp), few theta rows, and 19668
+    cells (full warps, the last one partly filled)."""
+    gpu, orc = _pair(*shape)
+    for _ in range(2):
+        gpu.step()
+        orc.step()
+        _same(gpu, orc)
+
+
+@pytest.mark.parametrize("opt", [{"radimp_start_with_bisect": 0}, {"radimp_scale_jacobian": 0}, {"radimp_lag_opac": 1},
+                                 {"radimp_allow_rad_ceiling": 0, "radimp_allow_entr_in_4dprim": 0},
+                                 {"radimp_opdamp_maxlevels": 1, "radimp_maxiter": 6}, {"synchrotron_bridge": 1}])
+def test_implicit_options(opt):
+    gpu, orc = _pair(32, 30, 1, **opt)
+    for _ in range(2):
+        gpu.step()
+        orc.step()
+        _same(gpu, orc)
+
+
+@pytest.mark.parametrize("nz", [1, 5])
+@pytest.mark.parametrize("bc", [(2, 2), (1, 2), (0, 1), (1, 0), (0, 0), (2, 1)])
+def test_ghost_fill_on_every_boundary(bc, nz):
+    """Faces and corners with periodic (0), copied (1) and PUFFY (2) x and y
+    boundaries, in 2D (whose corner means look across a period) and in 3D."""
+    gpu, orc = _pair(24, 20, nz, bc_x=bc[0], bc_y=bc[1], bc_z=0 if nz > 1 else 1)
+    gpu.setBc()
+    assert orc.lib.orc_sim_set_bc(orc.h) == 0
+    _same(gpu, orc)
+
+
+@pytest.mark.parametrize("shape", [(45, 45, 1), (64, 32, 1), (50, 41, 1), (160, 129, 1), (61, 40, 12)])
+def test_scalar_sums_around_the_fold_sizes(shape):
+    """Up to 2048 terms folded by one warp, more in chunks of 1024: 2025, 2048,
+    2050, 20640 and 29280 cells, shells inside the domain."""
+    gpu, orc = _pair(*shape)
+    a, b = gpu.scalars(0.1, 50.0, 15.0), orc.scalar_row(0.1, 50.0, 15.0)
+    for k in a:
+        assert np.float64(a[k]).view(np.uint64) == np.float64(b[k]).view(np.uint64), (k, a[k], b[k])
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 1777, 7200])
+def test_batch_forms_agree(n):
+    """Batches of one cell, around a warp, and around and above the device's
+    warps: the per-cell, persistent and sorted forms give the same bits."""
+    kc = koralcuda()
+    kc.lib()
+    opt = kc.puffy_options()
+    geom, dt, pp = kc.synth_implicit_cells(opt, n, 3)
+    ref = kc.implicit_batch(opt, geom, dt, pp, mode=0)
+    for mode in (1, 3, 5):
+        got = kc.implicit_batch(opt, geom, dt, pp, mode=mode)
+        assert np.array_equal(_bits(got[0]), _bits(ref[0])) and np.array_equal(got[1], ref[1])

@@ -1,7 +1,7 @@
 """The engine's lean implicit solve, W inversion and torus functions
 (koral-zig_b200/csrc/kc_implicit_lean.cuh, kc_u2p_lean.cuh, kc_init_lean.cuh)
-against the plain restatement of the reference (include/koral), bit for bit, on
-the host: the same source as the kernels, compiled by g++ with lean_check.cpp."""
+against the plain restatement of the reference (include/koral), and its parallel
+ordered fold (kc_fold.cuh) against the serial sum, bit for bit, on the host: the same source as the kernels, compiled by g++ with lean_check.cpp."""
 import os
 import subprocess
 
@@ -66,3 +66,9 @@ def test_torus_functions_are_bitwise_the_plain_ones(checker, spin):
     r = subprocess.run([checker, "init", str(spin)], check=True, capture_output=True, text=True)
     bad, n = (int(x) for x in r.stdout.split())
     assert bad == 0 and n > 100
+
+
+def test_parallel_fold_is_bitwise_the_serial_sum(checker):
+    r = subprocess.run([checker, "fold"], check=True, capture_output=True, text=True)
+    bad, mapped = (int(x) for x in r.stdout.split())
+    assert bad == 0 and mapped > 10000
