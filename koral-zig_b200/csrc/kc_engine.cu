@@ -59,7 +59,7 @@ struct kc_handle {
   cudaStream_t stream = nullptr;
   std::vector<void*> allocs;
   // stage buffers (koral/sim.zig:220)
-  double *ut0 = nullptr, *ut1 = nullptr, *ut2 = nullptr, *dut1 = nullptr, *dut2 = nullptr, *drt1 = nullptr,
+  double *ut0 = nullptr, *ut1 = nullptr, *ut2 = nullptr, *dut1 = nullptr, *drt1 = nullptr,
          *drt2 = nullptr, *uforget = nullptr, *staging = nullptr;
   int* flag_staging = nullptr;
   // step scalars (koral/sim.zig:237-293)
@@ -337,10 +337,11 @@ void launch_calc_u2p(kc_handle* h) {
                                                                 h->u2p_phi_fastest && gr.nz > 1);
   if (h->sp.do_fixups) {
     PassScope pf(h, KC_PASS_FIXUP);
+    const unsigned most = 8u * (unsigned)h->nsm, nb = nblk(ndom) < most ? nblk(ndom) : most;
     ++h->n_launch;
-    k_fixup_hd<<<nblk(ndom), TPB, 0, h->stream>>>(h->ds, h->dsc, h->sp.gam, pnc);
+    k_fixup_hd<<<nb, TPB, 0, h->stream>>>(h->ds, h->dsc, h->sp.gam, pnc);
     ++h->n_launch;
-    k_fixup_apply<<<nblk(ndom), TPB, 0, h->stream>>>(h->ds, h->dsc);
+    k_fixup_apply<<<nb, TPB, 0, h->stream>>>(h->ds, h->dsc);
   }
   launch_set_bc(h);
 }
@@ -504,7 +505,7 @@ void launch_face_fluxes(kc_handle* h) {
   a.fp32 = fp32_pieces(h->opt.precision);
   long dims[3] = {gr.nx, gr.ny, gr.nz};
   PassScope ps(h, KC_PASS_FLUXES);
-  for (int d = 0; d < 3; ++d) cudaMemsetAsync(h->ds.flb[d], 0, (size_t)NV * h->ds.nf[d] * 8, h->stream);
+  // faces outside the sweeps' ranges hold zeros from kc_create on
   for (int dim = 0; dim < 3; ++dim) {
     if (dims[dim] <= 1) continue;
     int c0 = dim == 0 ? 1 : 0, c1 = dim == 2 ? 1 : 2;
@@ -568,7 +569,6 @@ void launch_op_explicit(kc_handle* h, int dt_slot) {
 void launch_rijvisc(kc_handle* h, int dt_slot) {
   const DGrid& gr = h->gr;
   PassScope ps(h, KC_PASS_RADVISC);
-  cudaMemsetAsync(h->ds.rijvisc, 0, (size_t)16 * gr.nc * 8, h->stream);
   ViscArgs a;
   a.gam = h->sp.gam;
   a.dt_slot = dt_slot;
@@ -604,26 +604,20 @@ void launch_dynamo(kc_handle* h, int dt_slot) {
   launch_calc_u2p(h);
 }
 
-void launch_stage_deriv(kc_handle* h, double* dst, const double* a, const double* b, int delta) {
-  const DGrid& gr = h->gr;
-  PassScope ps(h, KC_PASS_STAGE);
-  ++h->n_launch;
-  k_stage_deriv<<<nblk((long)gr.nx * gr.ny * gr.nz, 256), 256, 0, h->stream>>>(h->ds, dst, a, b, delta);
-}
-void launch_stage_combine(kc_handle* h, double* dst, const double* a, int f1, const double* b, int f2,
-                          const double* c) {
-  const DGrid& gr = h->gr;
-  PassScope ps(h, KC_PASS_STAGE);
-  ++h->n_launch;
-  k_stage_combine<<<nblk((long)gr.nx * gr.ny * gr.nz, 256), 256, 0, h->stream>>>(h->ds, dst, a, f1, b, f2, c);
-}
 void copy_field(kc_handle* h, double* dst, const double* src) {
   PassScope ps(h, KC_PASS_STAGE);
   cudaMemcpyAsync(dst, src, (size_t)NV * h->gr.nc * 8, cudaMemcpyDeviceToDevice, h->stream);
 }
+// the stage kernels: one thread per domain cell
+template <class... A, class... B>
+void launch_stage(kc_handle* h, void (*kernel)(DevState, A...), B... args) {
+  PassScope ps(h, KC_PASS_STAGE);
+  ++h->n_launch;
+  kernel<<<nblk((long)h->gr.nx * h->gr.ny * h->gr.nz, 256), 256, 0, h->stream>>>(h->ds, args...);
+}
 
 // Coefficient slots of a step (run_step fills 0-3 before its first launch)
-enum { C_DT = 0, C_DT_GAM = 1, C_DT_1M2GAM = 2, C_DT_HALF = 3, NCOEF = 16 };
+enum : int { C_DT = 0, C_DT_GAM = 1, C_DT_1M2GAM = 2, C_DT_HALF = 3, NCOEF = 16 };
 // the slot holding v (bit-equal), appended and copied to the device if new;
 // a full table waits for the stream before it is reused (the host table is
 // pinned and read by copies when they run)
@@ -694,38 +688,26 @@ void enqueue_step(kc_handle* h) {
   // 1st implicit
   copy_field(h, h->ut0, u);
   launch_implicit(h, C_DT_GAM);
-  launch_stage_deriv(h, h->drt1, u, h->ut0, C_DT_GAM);
+  launch_stage(h, k_stage_deriv_copy, h->drt1, h->ut0, C_DT_GAM, h->ut1);
   // 1st explicit
-  copy_field(h, h->ut1, u);
   launch_calc_u2p(h);
   launch_do_correct(h);
   launch_set_bc(h);
   launch_op_explicit(h, C_DT);
   if (h->sp.dynamo) launch_dynamo(h, C_DT);
-  {
-    const DGrid& gr = h->gr;
-    PassScope ps(h, KC_PASS_STAGE);
-    ++h->n_launch;
-    k_copy_entropy_count<<<nblk((long)gr.nx * gr.ny * gr.nz, 256), 256, 0, h->stream>>>(h->ds);
-  }
-  launch_stage_deriv(h, h->dut1, u, h->ut1, C_DT);
-  launch_stage_combine(h, u, h->ut0, C_DT, h->dut1, C_DT_1M2GAM, h->drt1);
+  launch_stage(h, k_stage_mid, h->dut1, h->ut1, h->ut0, h->drt1, C_DT, C_DT_1M2GAM, h->uforget);
   // 2nd implicit
-  copy_field(h, h->uforget, u);
   launch_calc_u2p(h);
   launch_do_correct(h);
   launch_implicit(h, C_DT_GAM);
-  launch_stage_deriv(h, h->drt2, u, h->uforget, C_DT_GAM);
+  launch_stage(h, k_stage_deriv_copy, h->drt2, h->uforget, C_DT_GAM, h->ut2);
   // 2nd explicit
-  copy_field(h, h->ut2, u);
   launch_calc_u2p(h);
   launch_do_correct(h);
   launch_set_bc(h);
   launch_op_explicit(h, C_DT);
   if (h->sp.dynamo) launch_dynamo(h, C_DT);
-  launch_stage_deriv(h, h->dut2, u, h->ut2, C_DT);
-  launch_stage_combine(h, u, h->ut0, C_DT_HALF, h->dut1, C_DT_HALF, h->dut2);
-  launch_stage_combine(h, u, u, C_DT_HALF, h->drt1, C_DT_HALF, h->drt2);
+  launch_stage(h, k_stage_end, h->ut2, h->ut0, h->dut1, h->drt1, h->drt2, C_DT, C_DT_HALF);
   launch_calc_u2p(h);
   launch_do_correct(h);
   launch_set_bc(h);
@@ -950,7 +932,6 @@ int kc_create(const kc_grid* grid, const kc_options* opt, kc_handle** out) {
   h->ut1 = dalloc<double>(h, NV * nc, st);
   h->ut2 = dalloc<double>(h, NV * nc, st);
   h->dut1 = dalloc<double>(h, NV * nc, st);
-  h->dut2 = dalloc<double>(h, NV * nc, st);
   h->drt1 = dalloc<double>(h, NV * nc, st);
   h->drt2 = dalloc<double>(h, NV * nc, st);
   h->uforget = dalloc<double>(h, NV * nc, st);

@@ -221,37 +221,63 @@ __global__ void k_flags_to_aos(const int* __restrict__ soa, int* __restrict__ ao
 }
 
 // ---- stage arithmetic (koral/sim.zig:1586-1709) ------------------------------
-// dst = (1/delta) a + (-1/delta) b over the domain
-__global__ void k_stage_deriv(DevState s, double* dst, const double* a, const double* b, int delta_slot) {
+// Streaming passes over 13 components, bound by HBM (5.9 TB/s): the derivatives,
+// combinations and copies that follow each other are one pass each, 19 component
+// reads and writes a step less than one by one, and seven launches.
+
+// dst = (1/delta) u + (-1/delta) b over the domain, and the copy ut = u
+__global__ void k_stage_deriv_copy(DevState s, double* dst, const double* b, int delta_slot, double* ut) {
   const double delta = s.coef[delta_slot];
   Range r = {0, 0, 0, s.gr.nx, s.gr.ny, s.gr.nz};
   long ix, iy, iz;
   if (!range_cell(r, ix, iy, iz)) return;
-  long c = cidx(s.gr, ix, iy, iz);
-  double f1 = 1.0 / delta, f2 = -1.0 / delta;
-  long nc = s.gr.nc;
+  const long c = cidx(s.gr, ix, iy, iz), nc = s.gr.nc;
+  const double f1 = 1.0 / delta, f2 = -1.0 / delta;
 #pragma unroll
-  for (int iv = 0; iv < NV; ++iv) dst[iv * nc + c] = f1 * a[iv * nc + c] + f2 * b[iv * nc + c];
+  for (int iv = 0; iv < NV; ++iv) {
+    const double u = s.u[iv * nc + c];
+    dst[iv * nc + c] = f1 * u + f2 * b[iv * nc + c];
+    ut[iv * nc + c] = u;
+  }
 }
-// dst = a + f1 b + f2 cc over the domain
-__global__ void k_stage_combine(DevState s, double* dst, const double* a, int f1_slot, const double* b, int f2_slot,
-                                const double* cc) {
-  const double f1 = s.coef[f1_slot], f2 = s.coef[f2_slot];
+// The end of the first stage: dut1 = (u - ut1) / dt, then u and its copy uforget
+// = ut0 + dt dut1 + fc drt1, and the entropy flags' copy (C copy_entropycount)
+__global__ void k_stage_mid(DevState s, double* dut1, const double* ut1, const double* ut0, const double* drt1,
+                            int dt_slot, int fc_slot, double* uforget) {
+  const double dt = s.coef[dt_slot], fc = s.coef[fc_slot];
   Range r = {0, 0, 0, s.gr.nx, s.gr.ny, s.gr.nz};
   long ix, iy, iz;
   if (!range_cell(r, ix, iy, iz)) return;
-  long c = cidx(s.gr, ix, iy, iz);
-  long nc = s.gr.nc;
+  const long c = cidx(s.gr, ix, iy, iz), nc = s.gr.nc;
+  const double f1 = 1.0 / dt, f2 = -1.0 / dt;
 #pragma unroll
-  for (int iv = 0; iv < NV; ++iv) dst[iv * nc + c] = a[iv * nc + c] + f1 * b[iv * nc + c] + f2 * cc[iv * nc + c];
+  for (int iv = 0; iv < NV; ++iv) {
+    const long k = iv * nc + c;
+    const double d = f1 * s.u[k] + f2 * ut1[k];
+    const double u = ut0[k] + dt * d + fc * drt1[k];
+    dut1[k] = d;
+    s.u[k] = u;
+    uforget[k] = u;
+  }
+  s.flags[2 * nc + c] = s.flags[0 * nc + c];
 }
-// flags entropy3 = entropy (C copy_entropycount)
-__global__ void k_copy_entropy_count(DevState s) {
+// The end of the step: dut2 = (u - ut2) / dt, u = ut0 + h dut1 + h dut2, then
+// u = u + h drt1 + h drt2
+__global__ void k_stage_end(DevState s, const double* ut2, const double* ut0, const double* dut1, const double* drt1,
+                            const double* drt2, int dt_slot, int h_slot) {
+  const double dt = s.coef[dt_slot], h = s.coef[h_slot];
   Range r = {0, 0, 0, s.gr.nx, s.gr.ny, s.gr.nz};
   long ix, iy, iz;
   if (!range_cell(r, ix, iy, iz)) return;
-  long c = cidx(s.gr, ix, iy, iz);
-  s.flags[2 * s.gr.nc + c] = s.flags[0 * s.gr.nc + c];
+  const long c = cidx(s.gr, ix, iy, iz), nc = s.gr.nc;
+  const double f1 = 1.0 / dt, f2 = -1.0 / dt;
+#pragma unroll
+  for (int iv = 0; iv < NV; ++iv) {
+    const long k = iv * nc + c;
+    const double d = f1 * s.u[k] + f2 * ut2[k];
+    const double u = ut0[k] + h * dut1[k] + h * d;
+    s.u[k] = u + h * drt1[k] + h * drt2[k];
+  }
 }
 // C update_entropy (koral/sim.zig:1683)
 __global__ void __launch_bounds__(128) k_update_entropy(DevState s, double gam) {
@@ -321,11 +347,8 @@ __global__ void __launch_bounds__(128, KC_U2P_MIN_BLOCKS) k_u2p(DevState s, DevS
 
 // cell_fixup(FIXUP_U2PMHD), pass 1: flagged cells average their non-flagged
 // in-domain neighbours into the staging buffers (koral/sim.zig:1067)
-__global__ void __launch_bounds__(128) k_fixup_hd(DevState s, DevScalars* sc, double gam, int polar_nc) {
-  if (!sc->any_hd) return;
-  Range r = {0, 0, 0, s.gr.nx, s.gr.ny, s.gr.nz};
-  long ix, iy, iz;
-  if (!range_cell(r, ix, iy, iz)) return;
+// (both passes over few blocks: most u2p passes flag no cell and they return)
+__device__ void fixup_hd_cell(const DevState& s, double gam, int polar_nc, long ix, long iy, long iz) {
   long nc = s.gr.nc, c = cidx(s.gr, ix, iy, iz);
   if (polar_nc > 0 && (iy < polar_nc || iy > s.gr.ny - polar_nc - 1)) return;
   const int* fhd = s.flags + 3 * nc;
@@ -361,20 +384,26 @@ __global__ void __launch_bounds__(128) k_fixup_hd(DevState s, DevScalars* sc, do
   // neighbour tests of concurrent threads and is cleared in pass 2
   s.flags[3 * nc + c] = fhd[c] | 0x40000000;
 }
-// pass 2: copy the staged cells back
-__global__ void k_fixup_apply(DevState s, DevScalars* sc) {
+__global__ void __launch_bounds__(128) k_fixup_hd(DevState s, DevScalars* sc, double gam, int polar_nc) {
   if (!sc->any_hd) return;
-  Range r = {0, 0, 0, s.gr.nx, s.gr.ny, s.gr.nz};
-  long ix, iy, iz;
-  if (!range_cell(r, ix, iy, iz)) return;
-  long nc = s.gr.nc, c = cidx(s.gr, ix, iy, iz);
-  int f = s.flags[3 * nc + c];
-  if (!(f & 0x40000000)) return;
-  s.flags[3 * nc + c] = f & ~0x40000000;
+  const long nx = s.gr.nx, ny = s.gr.ny, n = nx * ny * s.gr.nz;
+  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
+    fixup_hd_cell(s, gam, polar_nc, t % nx, t / nx % ny, t / nx / ny);
+}
+// pass 2: copy the staged cells back
+__global__ void __launch_bounds__(128) k_fixup_apply(DevState s, DevScalars* sc) {
+  if (!sc->any_hd) return;
+  const long nx = s.gr.nx, ny = s.gr.ny, nc = s.gr.nc, n = nx * ny * s.gr.nz;
+  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
+    const long c = cidx(s.gr, t % nx, t / nx % ny, t / nx / ny);
+    const int f = s.flags[3 * nc + c];
+    if (!(f & 0x40000000)) continue;
+    s.flags[3 * nc + c] = f & ~0x40000000;
 #pragma unroll
-  for (int iv = 0; iv < NV; ++iv) {
-    s.p[iv * nc + c] = s.fix_p[iv * nc + c];
-    s.u[iv * nc + c] = s.fix_u[iv * nc + c];
+    for (int iv = 0; iv < NV; ++iv) {
+      s.p[iv * nc + c] = s.fix_p[iv * nc + c];
+      s.u[iv * nc + c] = s.fix_u[iv * nc + c];
+    }
   }
 }
 
@@ -885,6 +914,7 @@ __global__ void __launch_bounds__(128, KC_FLUX_MIN_BLOCKS) k_face_flux(DevState 
   if (!e) e = face_state(s, sc, a, dim, pR, geo, c, cm, ffr, uR);
   if (e) {
     set_err(sc, e, c);
+    for (int iv = 0; iv < NV; ++iv) s.flb[dim][iv * s.nf[dim] + face_index(s.gr, dim, cf[0], cf[1], cf[2])] = 0.0;
     return;
   }
   double ag = kmath::fmax(s.amax[(long)dim * nc + c], s.amax[(long)dim * nc + cm]);
@@ -1001,6 +1031,7 @@ __global__ void __launch_bounds__(128, KC_FLUX_MIN_BLOCKS) k_face_flux_tiled(Dev
   if (!e) e = face_state(s, sc, a, dim, pR, geo, c, cm, ffr, uR);
   if (e) {
     set_err(sc, e, c);
+    for (int iv = 0; iv < NV; ++iv) s.flb[dim][iv * s.nf[dim] + face_index(s.gr, dim, cf[0], cf[1], cf[2])] = 0.0;
     return;
   }
   const double ag = kmath::fmax(s.amax[(long)dim * nc + c], s.amax[(long)dim * nc + cm]);
