@@ -299,31 +299,35 @@ int sync_check(kc_handle* h, const char* what) {
   return KC_OK;
 }
 
-BcArgs bc_args(kc_handle* h) {
-  BcArgs a;
-  a.bc[0] = h->sp.bc[0];
-  a.bc[1] = h->sp.bc[1];
-  a.bc[2] = h->sp.bc[2];
-  a.gam = h->sp.gam;
-  return a;
-}
-
-// C set_bc (koral/sim/bc.zig:40)
+// C set_bc (koral/sim/bc.zig:40): faces and corners in one launch
 void launch_set_bc(kc_handle* h) {
   PassScope ps(h, KC_PASS_BC);
   const DGrid& gr = h->gr;
-  BcArgs a = bc_args(h);
-  cudaStream_t st = h->stream;
-  const unsigned bx = nblk(2L * gr.ngx * gr.ny * gr.nz), by = nblk(2L * gr.ngy * gr.nx * gr.nz),
-                 bz = nblk(2L * gr.ngz * gr.nx * gr.ny);
+  const long ng = gr.ng;
+  const bool corners = gr.nx > 1 && gr.ny > 1;
+  const long n = !corners ? 0 : gr.nz == 1 ? 4 * 2 * ng : 4L * ((long)gr.nx + gr.ny + gr.nz) * 2 * ng + 8 * ng * ng * ng;
+  BcArgs a;
+  for (int k = 0; k < 3; ++k) a.bc[k] = h->sp.bc[k];
+  a.gam = h->sp.gam;
+  a.b1 = nblk(2L * gr.ngx * gr.ny * gr.nz);
+  a.b2 = a.b1 + nblk(2L * gr.ngy * gr.nx * gr.nz);
+  a.b3 = a.b2 + nblk(2L * gr.ngz * gr.nx * gr.ny);
   ++h->n_launch;
-  k_bc_faces<<<bx + by + bz, TPB, 0, st>>>(h->ds, h->dsc, a, bx, bx + by);
-  if (gr.nx > 1 && gr.ny > 1) {
-    const long ng = gr.ng;
-    const long n = gr.nz == 1 ? 4 * 2 * ng : 4L * ((long)gr.nx + gr.ny + gr.nz) * 2 * ng + 8 * ng * ng * ng;
-    ++h->n_launch;
-    k_corners<<<nblk(n, 64), 64, 0, st>>>(h->ds, a);
-  }
+  k_set_bc<<<a.b3 + nblk(n), TPB, 0, h->stream>>>(h->ds, h->dsc, a);
+}
+
+// Cells that each warp of the implicit and u2p passes carries: all 32 lanes once the
+// grid has 32 cells for four warps an SM, a smaller power of two on smaller grids,
+// whose passes last as long as their slowest warp (the union of its lanes' paths;
+// one cell is a serial chain of dependent FP64 operations either way). Measured,
+// ladder and u2p per launch: 32x30 176 and 52 us with 32, 161 and 42 with 2, 162
+// with 8; 32x30x4 218 and 39 with 32, 190 and 35 with 8, 214 with 7; 101x75 196 and
+// 46 with 32, 189 with 16, 215 with 8, 316 with 4.
+int solve_lanes(long ncell, int nsm) {
+  const long need = (ncell + 4L * nsm - 1) / (4L * nsm);
+  int l = 1;
+  while (l < need && l < 32) l *= 2;
+  return l;
 }
 
 void launch_calc_u2p(kc_handle* h) {
@@ -333,8 +337,9 @@ void launch_calc_u2p(kc_handle* h) {
   PassScope ps(h, KC_PASS_U2P);
   cudaMemsetAsync(&h->dsc->any_hd, 0, sizeof(int), h->stream);
   ++h->n_launch;
-  k_u2p<<<nblk(ndom, h->tpb_u2p), h->tpb_u2p, 0, h->stream>>>(h->ds, h->dsc, h->sp.gam, h->sp.fl, h->sp.rp, pnc,
-                                                                h->u2p_phi_fastest && gr.nz > 1);
+  const int lanes = solve_lanes(ndom, h->nsm);
+  k_u2p<<<nblk((ndom + lanes - 1) / lanes * 32, h->tpb_u2p), h->tpb_u2p, 0, h->stream>>>(
+      h->ds, h->dsc, h->sp.gam, h->sp.fl, h->sp.rp, pnc, h->u2p_phi_fastest && gr.nz > 1, lanes);
   if (h->sp.do_fixups) {
     PassScope pf(h, KC_PASS_FIXUP);
     const unsigned most = 8u * (unsigned)h->nsm, nb = nblk(ndom) < most ? nblk(ndom) : most;
@@ -381,16 +386,6 @@ int ensure_split(kc_handle* h) {
   return KC_OK;
 }
 
-// Cells that each warp of the implicit pass carries: all 32 lanes once the grid has
-// 32 cells for four warps an SM, fewer on smaller grids, whose passes last as long
-// as their slowest warp (the union of its lanes' paths; one solve is a serial
-// chain of dependent FP64 operations either way). Measured, ladder per launch:
-// 32x30 171 us with 32, 156 with 2 to 8, 162 with 1; 32x30x4 210 with 32, 179 with
-// 4, 291 with 2; 101x75 187 with 32, 189 with 16, 286 with 4.
-int implicit_lanes(long ncell, int nsm) {
-  const long l = (ncell + 4L * nsm - 1) / (4L * nsm);
-  return l > 32 ? 32 : (int)l;
-}
 void launch_implicit(kc_handle* h, int dt_slot) {
   const DGrid& gr = h->gr;
   ImplArgs a;
@@ -453,7 +448,7 @@ void launch_implicit(kc_handle* h, int dt_slot) {
   cudaStream_t st = h->stream;
   // the AoS staging array is free inside a step: 8 doubles and an int per cell of its NV doubles
   const WarmBuf wb = {h->staging, (int*)(h->staging + 8 * ndom), ndom};
-  const int lanes = implicit_lanes(ndom, h->nsm);
+  const int lanes = solve_lanes(ndom, h->nsm);
   const long nthread = (ndom + lanes - 1) / lanes * 32;
   h->n_launch += 2;
   if (x.guess)
@@ -461,13 +456,18 @@ void launch_implicit(kc_handle* h, int dt_slot) {
                                                                                                     x.guess, lanes);
   else
     k_implicit_warm<<<nblk(nthread, KC_WARM_TPB), KC_WARM_TPB, 0, st>>>(h->ds, a, wb, lanes);
-  // the learned-guess and harvest forms in the default block
-  const int nt = extra ? KC_IMPLICIT_TPB : h->tpb_implicit;
+  // the learned-guess and harvest forms in the default block. A grid of few warps
+  // leaves the other warps' registers unused, so it runs the 255-register
+  // instance in small blocks spread over the SMs, whatever the block size set
+  // (32x30: 156 us a launch in blocks of 64, 166 of 256; 226 in the 168-register
+  // instance)
+  const bool few = !extra && nthread <= 8L * 32 * h->nsm;
+  const int nt = extra ? KC_IMPLICIT_TPB : few ? 64 : h->tpb_implicit;
   const unsigned nb = nblk(nthread, nt);
   const size_t sm = SharedCell::bytes(nt);
   if (h->hcap > 0) k_implicit_ext<true><<<nb, nt, sm, st>>>(h->ds, h->dsc, a, wb, x, lanes);
   else if (extra) k_implicit_ext<false><<<nb, nt, sm, st>>>(h->ds, h->dsc, a, wb, x, lanes);
-  else if (nt == 256) k_implicit<256><<<nb, nt, sm, st>>>(h->ds, h->dsc, a, wb, lanes);
+  else if (few || nt == 256) k_implicit<256><<<nb, nt, sm, st>>>(h->ds, h->dsc, a, wb, lanes);
   else if (nt == 512) k_implicit<512><<<nb, nt, sm, st>>>(h->ds, h->dsc, a, wb, lanes);
   else k_implicit<384><<<nb, nt, sm, st>>>(h->ds, h->dsc, a, wb, lanes);
 }

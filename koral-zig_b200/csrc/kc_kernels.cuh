@@ -48,18 +48,6 @@ __device__ __forceinline__ unsigned long long dbits(double x) { return (unsigned
 struct Range {
   long x0, y0, z0, nx, ny, nz;
 };
-// The domain cell of this thread with phi (z) fastest: the cells of a warp then
-// share (r, theta), and on an axisymmetric torus they take nearly the same path
-// through a per-cell solver (the implicit solve, the u2p inversion).
-__device__ __forceinline__ bool domain_cell_phi_fastest(const DGrid& gr, long& ix, long& iy, long& iz) {
-  long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long)gr.nx * gr.ny * gr.nz) return false;
-  iz = t % gr.nz;
-  long q = t / gr.nz;
-  ix = q % gr.nx;
-  iy = q / gr.nx;
-  return true;
-}
 __device__ __forceinline__ bool range_cell(const Range& r, long& ix, long& iy, long& iz) {
   long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   long n = r.nx * r.ny * r.nz;
@@ -300,13 +288,20 @@ __global__ void __launch_bounds__(128) k_update_entropy(DevState s, double gam) 
 // ---- u2p (koral/sim.zig:924-1000) --------------------------------------------
 __global__ void __launch_bounds__(128, KC_U2P_MIN_BLOCKS) k_u2p(DevState s, DevScalars* sc, double gam, const __grid_constant__ FloorParams fl,
                                              const __grid_constant__ RadParams rp,
-                                             int polar_nc, int phi_fastest) {
-  Range r = {0, 0, 0, s.gr.nx, s.gr.ny, s.gr.nz};
+                                             int polar_nc, int phi_fastest, int lanes) {
+  const long nx = s.gr.nx, ny = s.gr.ny, nz = s.gr.nz;
+  const int lane = threadIdx.x & 31;
+  const long t = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32 * lanes + lane;
+  if (lane >= lanes || t >= nx * ny * nz) return;
   long ix, iy, iz;
   if (phi_fastest) {
-    if (!domain_cell_phi_fastest(s.gr, ix, iy, iz)) return;
-  } else if (!range_cell(r, ix, iy, iz)) {
-    return;
+    iz = t % nz;
+    ix = t / nz % nx;
+    iy = t / nz / nx;
+  } else {
+    ix = t % nx;
+    iy = t / nx % ny;
+    iz = t / nx / ny;
   }
   long c = cidx(s.gr, ix, iy, iz), nc = s.gr.nc;
   double uu[NV], pp[NV];
@@ -479,20 +474,15 @@ __device__ int puffy_bc_cell(const DevState& s, long ix, long iy, long iz, int f
   return E_OK;
 }
 
-__device__ void bc_cell(const DevState& s, DevScalars* sc, long ix, long iy, long iz, int face, const int bc[3],
-                        double gam) {
-  int axis = face / 2;
-  int kind = bc[axis];
-  long nc = s.gr.nc;
-  double pp[NV];
-  if (kind == KC_BC_PUFFY) {
-    int e = puffy_bc_cell(s, ix, iy, iz, face, pp);
-    if (e) {
-      set_err(sc, e, cidx(s.gr, ix, iy, iz));
-      return;
-    }
-  } else {
-    long iix = ix, iiy = iy, iiz = iz, nx = s.gr.nx, ny = s.gr.ny, nz = s.gr.nz;
+// The primitives of a face ghost (face: 2 axis + high), or of a domain cell (face 6)
+__device__ __forceinline__ int ghost_prims(const DevState& s, long ix, long iy, long iz, int face, const int bc[3],
+                                           double pp[NV]) {
+  const long nc = s.gr.nc, nx = s.gr.nx, ny = s.gr.ny, nz = s.gr.nz;
+  const int axis = face >> 1;
+  long iix = ix, iiy = iy, iiz = iz;
+  if (axis < 3) {
+    const int kind = bc[axis];
+    if (kind == KC_BC_PUFFY) return puffy_bc_cell(s, ix, iy, iz, face, pp);
     if (axis == 0) {
       if (kind == KC_BC_PERIODIC) {
         if (ix < 0) iix = ix + nx;
@@ -520,168 +510,185 @@ __device__ void bc_cell(const DevState& s, DevScalars* sc, long ix, long iy, lon
         if (iz > nz - 1) iiz = nz - 1;
       }
     }
-    load_cell(s.p, nc, cidx(s.gr, iix, iiy, iiz), pp);
   }
-  Geom g;
-  geom_cell(s, ix, iy, iz, g);
-  double uu[NV];
-  p2u(pp, uu, g, gam);
-  long c = cidx(s.gr, ix, iy, iz);
-  store_cell(s.p, nc, c, pp);
-  store_cell(s.u, nc, c, uu);
+  load_cell(s.p, nc, cidx(s.gr, iix, iiy, iiz), pp);
+  return E_OK;
 }
-
 struct BcArgs {
   int bc[3];
   double gam;
+  unsigned b1, b2, b3;  // the blocks where the y faces, the z faces and the corners begin
 };
-// The ghost faces of all axes in one launch: they read domain cells only, so the
-// three axes are independent. Bound by launch latency and one chain of loads and
-// p2u per cell: 8 us on small grids, where three launches took 18. Blocks [0, b1) fill the x faces, [b1, b2) the y
-// faces, the rest the z faces; thread -> (ghost layer i, two transverse indices).
-__global__ void __launch_bounds__(128, KC_BC_MIN_BLOCKS) k_bc_faces(DevState s, DevScalars* sc, BcArgs a, unsigned b1,
-                                                                    unsigned b2) {
-  const int axis = blockIdx.x < b1 ? 0 : blockIdx.x < b2 ? 1 : 2;
-  const long t = (long)(blockIdx.x - (axis == 0 ? 0u : axis == 1 ? b1 : b2)) * blockDim.x + threadIdx.x;
-  const long nx = s.gr.nx, ny = s.gr.ny, nz = s.gr.nz;
-  if (axis == 0) {
-    const long ng = s.gr.ngx;
-    if (t >= 2 * ng * ny * nz) return;
-    const long side = t % 2, q = t / 2;
-    const long i = 1 + q % ng, r = q / ng;
-    const long iy = r % ny, iz = r / ny;
-    if (side == 0) bc_cell(s, sc, -i, iy, iz, 0, a.bc, a.gam);
-    else bc_cell(s, sc, nx - 1 + i, iy, iz, 1, a.bc, a.gam);
-  } else if (axis == 1) {
-    const long ng = s.gr.ngy;
-    if (t >= 2 * ng * nx * nz) return;
-    const long ix = t % nx, q = t / nx;
-    const long side = q % 2, r = q / 2;
-    const long i = 1 + r % ng, iz = r / ng;
-    if (side == 0) bc_cell(s, sc, ix, -i, iz, 2, a.bc, a.gam);
-    else bc_cell(s, sc, ix, ny - 1 + i, iz, 3, a.bc, a.gam);
-  } else {
-    const long ng = s.gr.ngz;
-    if (t >= 2 * ng * nx * ny) return;
-    const long ix = t % nx, q = t / nx;
-    const long iy = q % ny, r = q / ny;
-    const long side = r % 2, i = 1 + r / 2;
-    if (side == 0) bc_cell(s, sc, ix, iy, -i, 4, a.bc, a.gam);
-    else bc_cell(s, sc, ix, iy, nz - 1 + i, 5, a.bc, a.gam);
-  }
-}
-
-__device__ void p2u_cell(const DevState& s, long ix, long iy, long iz, double gam) {
-  long nc = s.gr.nc, c = cidx(s.gr, ix, iy, iz);
-  double pp[NV], uu[NV];
-  load_cell(s.p, nc, c, pp);
-  Geom g;
-  geom_cell(s, ix, iy, iz, g);
-  p2u(pp, uu, g, gam);
-  store_cell(s.u, nc, c, uu);
-}
-__device__ void copy_p_cell(const DevState& s, long dx, long dy, long dz, long sx_, long sy_, long sz_) {
-  long nc = s.gr.nc, d = cidx(s.gr, dx, dy, dz), c = cidx(s.gr, sx_, sy_, sz_);
-#pragma unroll
-  for (int iv = 0; iv < NV; ++iv) s.p[iv * nc + d] = s.p[iv * nc + c];
-}
-__device__ void avg_p_cell(const DevState& s, const long d[3], const long a[3], const long b[3]) {
-  long nc = s.gr.nc, cd = cidx(s.gr, d[0], d[1], d[2]), ca = cidx(s.gr, a[0], a[1], a[2]),
-       cb = cidx(s.gr, b[0], b[1], b[2]);
-  double v[NV];
-  for (int iv = 0; iv < NV; ++iv) v[iv] = 0.5 * (s.p[iv * nc + ca] + s.p[iv * nc + cb]);
-  store_cell(s.p, nc, cd, v);
-}
-
-// The corner ghosts, one thread per cell. The reference fills them in groups whose
-// later members read cells that earlier ones wrote; each such cell is a copy of a
-// face ghost, so a thread reads the face ghost itself and all are independent.
-//
-// Around an edge of the (pa, pb) plane (bc.zig:256 in 2D, :404 in 3D) a corner has
-// 2 (ng-1) strip cells, (a outer, b first) and (a first, b outer), copies of the
-// face ghosts beside them, the mean of its two adjoining face ghosts at (first,
-// first), and at (second, second) the mean of two strip cells.
-__device__ __forceinline__ void tube_cell(int pa, int pb, int pc, long av, long bv, long cv, long o[3]) {
+// a ghost cell d and the one or two cells whose primitives (their mean) it takes
+struct GhostTask {
+  long d[3], x[2][3];
+  int face[2];
+  int n;  // sources; 0: no such cell
+};
+__device__ __forceinline__ void ghost_at(long o[3], int pa, int pb, int pc, long av, long bv, long cv) {
   o[pa] = av;
   o[pb] = bv;
   o[pc] = cv;
 }
-// per_a, per_b: a 2D grid periodic in that direction takes the means' sources
-// from across it (bc.zig:256); a 3D edge never does
-__device__ void corner_edge_cell(const DevState& s, double gam, int pa, int pb, int pc, long cc, int tube, long task,
-                                 bool per_a, bool per_b) {
-  const long dims[3] = {s.gr.nx, s.gr.ny, s.gr.nz};
-  const long ng = s.gr.ng, na = dims[pa], nb = dims[pb];
-  const bool a_hi = tube & 2, b_hi = tube & 1;
+// Thread t of the faces of `axis`: (ghost layer i, two transverse indices)
+__device__ __forceinline__ void face_task(const DGrid& gr, int axis, long t, GhostTask& g) {
+  const long nx = gr.nx, ny = gr.ny, nz = gr.nz;
+  const long ng = axis == 0 ? gr.ngx : axis == 1 ? gr.ngy : gr.ngz;
+  const long n = axis == 0 ? nx : axis == 1 ? ny : nz;
+  g.n = 0;
+  if (t >= 2 * ng * (nx * ny * nz / n)) return;
+  long side, i, u, v;  // u, v: the transverse indices
+  if (axis == 0) {
+    side = t % 2;
+    i = t / 2 % ng;
+    u = t / 2 / ng % ny;
+    v = t / 2 / ng / ny;
+  } else if (axis == 1) {
+    u = t % nx;
+    side = t / nx % 2;
+    i = t / nx / 2 % ng;
+    v = t / nx / 2 / ng;
+  } else {
+    u = t % nx;
+    v = t / nx % ny;
+    side = t / nx / ny % 2;
+    i = t / nx / ny / 2;
+  }
+  const int pu = axis == 0 ? 1 : 0, pv = axis == 2 ? 1 : 2;
+  ghost_at(g.d, axis, pu, pv, side ? n + i : -1 - i, u, v);
+  for (int k = 0; k < 3; ++k) g.x[0][k] = g.d[k];
+  g.face[0] = 2 * axis + (int)side;
+  g.n = 1;
+}
+// A corner ghost around an edge of the (pa, pb) plane (bc.zig:256 in 2D, :404 in
+// 3D): 2 (ng-1) strip cells, (a outer, b first) and (a first, b outer), copies of
+// the face ghosts beside them; at (first, first) the mean of the two adjoining face
+// ghosts, at (second, second) the mean of two strip cells, which are copies of face
+// ghosts again. per_a, per_b: a 2D grid periodic in that direction takes the means'
+// sources from across it; a 3D edge never does.
+__device__ __forceinline__ void edge_task(const DGrid& gr, int pa, int pb, int pc, long cc, int tube, long task, bool per_a,
+                                          bool per_b, GhostTask& g) {
+  const long dims[3] = {gr.nx, gr.ny, gr.nz};
+  const long ng = gr.ng, na = dims[pa], nb = dims[pb];
+  const int a_hi = tube >> 1, b_hi = tube & 1;
   const long a_edge = a_hi ? na - 1 : 0, b_edge = b_hi ? nb - 1 : 0;
   const long nstrip = 2 * (ng - 1);
-  long d[3], x[3], y[3];
   if (task < nstrip) {
     const long i = task >> 1;
+    g.n = 1;
     if ((task & 1) == 0) {
       const long a_out = a_hi ? na + i + 1 : -ng + i;
-      tube_cell(pa, pb, pc, a_out, b_hi ? nb : -1, cc, d);
-      tube_cell(pa, pb, pc, a_out, b_edge, cc, x);
+      ghost_at(g.d, pa, pb, pc, a_out, b_hi ? nb : -1, cc);
+      ghost_at(g.x[0], pa, pb, pc, a_out, b_edge, cc);
+      g.face[0] = 2 * pa + a_hi;
     } else {
       const long b_out = b_hi ? nb + i + 1 : -ng + i;
-      tube_cell(pa, pb, pc, a_hi ? na : -1, b_out, cc, d);
-      tube_cell(pa, pb, pc, a_edge, b_out, cc, x);
+      ghost_at(g.d, pa, pb, pc, a_hi ? na : -1, b_out, cc);
+      ghost_at(g.x[0], pa, pb, pc, a_edge, b_out, cc);
+      g.face[0] = 2 * pb + b_hi;
     }
-    copy_p_cell(s, d[0], d[1], d[2], x[0], x[1], x[2]);
-  } else {
-    const long k = task - nstrip;  // 0: (first, first), 1: (second, second)
-    const long a_g = a_hi ? na + k : -1 - k, b_g = b_hi ? nb + k : -1 - k;
-    tube_cell(pa, pb, pc, a_g, b_g, cc, d);
-    if (per_a) {  // both sources the b ghost across the periodic a
-      tube_cell(pa, pb, pc, a_hi ? k : na - 1 - k, b_g, cc, x);
-      tube_cell(pa, pb, pc, a_hi ? k : na - 1 - k, b_g, cc, y);
-    } else if (per_b) {
-      tube_cell(pa, pb, pc, a_g, b_hi ? k : nb - 1 - k, cc, x);
-      tube_cell(pa, pb, pc, a_g, b_hi ? k : nb - 1 - k, cc, y);
-    } else {
-      // k = 1: the strip cells (a second, b first), (a first, b second) are
-      // copies of these
-      tube_cell(pa, pb, pc, a_g, b_edge, cc, x);
-      tube_cell(pa, pb, pc, a_edge, b_g, cc, y);
-    }
-    avg_p_cell(s, d, x, y);
+    return;
   }
-  p2u_cell(s, d[0], d[1], d[2], gam);
+  const long k = task - nstrip;  // 0: (first, first), 1: (second, second)
+  const long a_g = a_hi ? na + k : -1 - k, b_g = b_hi ? nb + k : -1 - k;
+  ghost_at(g.d, pa, pb, pc, a_g, b_g, cc);
+  g.n = 2;
+  ghost_at(g.x[0], pa, pb, pc, a_g, b_edge, cc);
+  g.face[0] = 2 * pa + a_hi;
+  ghost_at(g.x[1], pa, pb, pc, a_edge, b_g, cc);
+  g.face[1] = 2 * pb + b_hi;
+  if (per_a) {  // both sources the b ghost across the periodic a
+    ghost_at(g.x[0], pa, pb, pc, a_hi ? k : na - 1 - k, b_g, cc);
+    g.face[0] = g.face[1];
+    ghost_at(g.x[1], pa, pb, pc, a_hi ? k : na - 1 - k, b_g, cc);
+  } else if (per_b) {
+    ghost_at(g.x[1], pa, pb, pc, a_g, b_hi ? k : nb - 1 - k, cc);
+    g.face[1] = g.face[0];
+    ghost_at(g.x[0], pa, pb, pc, a_g, b_hi ? k : nb - 1 - k, cc);
+  }
 }
 // 2D: the four corners. 3D: the edges along z, y and x over the domain, and the 8
 // corner cubes (bc.zig:457), copies of the domain's corner cells (the reference's
 // edges also run through the cubes, which then overwrite them).
-__global__ void __launch_bounds__(64) k_corners(DevState s, BcArgs a) {
-  long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long nx = s.gr.nx, ny = s.gr.ny, nz = s.gr.nz, ng = s.gr.ng;
-  const long ntask = 2 * ng;
+__device__ __forceinline__ void corner_task(const DGrid& gr, const int bc[3], long t, GhostTask& g) {
+  const long nx = gr.nx, ny = gr.ny, nz = gr.nz, ng = gr.ng, ntask = 2 * ng;
+  g.n = 0;
   if (nz == 1) {
     if (t >= 4 * ntask) return;
-    // corner bit 0: x high, bit 1: y high
-    const int corner = (int)(t / ntask);
-    const int tube = (corner & 1) * 2 + (corner >> 1);
-    const bool px = a.bc[0] == KC_BC_PERIODIC, py = a.bc[1] == KC_BC_PERIODIC;
-    corner_edge_cell(s, a.gam, 0, 1, 2, 0, tube, t % ntask, px, py);
+    const int corner = (int)(t / ntask);  // bit 0: x high, bit 1: y high
+    edge_task(gr, 0, 1, 2, 0, (corner & 1) * 2 + (corner >> 1), t % ntask, bc[0] == KC_BC_PERIODIC,
+              bc[1] == KC_BC_PERIODIC, g);
     return;
   }
-  for (int e = 0; e < 3; ++e) {
-    const int pa = e == 2 ? 1 : 0, pb = e == 0 ? 1 : 2, pc = 2 - e;
-    const long len = pc == 0 ? nx : pc == 1 ? ny : nz;
-    if (t < 4 * len * ntask) {
-      const long q = t / ntask;
-      corner_edge_cell(s, a.gam, pa, pb, pc, q % len, (int)(q / len), t % ntask, false, false);
-      return;
+  long cc = t / ntask;  // over the 4 nz, 4 ny and 4 nx slices of the three edge groups
+  if (cc < 4 * (nx + ny + nz)) {
+    int pa = 0, pb = 1, pc = 2;
+    long len = nz;
+    if (cc >= 4 * nz) {
+      cc -= 4 * nz;
+      pb = 2;
+      pc = 1;
+      len = ny;
+      if (cc >= 4 * ny) {
+        cc -= 4 * ny;
+        pa = 1;
+        pc = 0;
+        len = nx;
+      }
     }
-    t -= 4 * len * ntask;
+    edge_task(gr, pa, pb, pc, cc % len, (int)(cc / len), t % ntask, false, false, g);
+    return;
   }
+  t -= 4 * (nx + ny + nz) * ntask;
   const long per = ng * ng * ng;
   if (t >= 8 * per) return;
   const int cube = (int)(t / per);
   t %= per;
   const bool xh = cube & 1, yh = cube & 2, zh = cube & 4;
-  const long ix = (xh ? nx : -ng) + t % ng, iy = (yh ? ny : -ng) + (t / ng) % ng, iz = (zh ? nz : -ng) + t / (ng * ng);
-  copy_p_cell(s, ix, iy, iz, xh ? nx - 1 : 0, yh ? ny - 1 : 0, zh ? nz - 1 : 0);
-  p2u_cell(s, ix, iy, iz, a.gam);
+  g.d[0] = (xh ? nx : -ng) + t % ng;
+  g.d[1] = (yh ? ny : -ng) + t / ng % ng;
+  g.d[2] = (zh ? nz : -ng) + t / (ng * ng);
+  g.x[0][0] = xh ? nx - 1 : 0;
+  g.x[0][1] = yh ? ny - 1 : 0;
+  g.x[0][2] = zh ? nz - 1 : 0;
+  g.face[0] = 6;
+  g.n = 1;
+}
+// Every ghost cell in one launch. The reference fills faces, then corners in
+// groups whose later members read cells that earlier ones wrote; but a face ghost
+// is a function of domain cells, and a corner ghost a copy or a mean of face
+// ghosts, so a corner's thread forms those face ghosts itself and no cell waits
+// for another. Bound on small grids by launch latency and one cell's chain of
+// loads, transforms and p2u: 8.9 us a launch (8.8 and 8.4 us as a face and a
+// corner launch, 22 and twice 6.5 us in 2D one by one; ten launches in 3D). On the
+// 192x180x64 wedge 85 us (89; 138), with 241 registers; 94 with 168.
+__global__ void __launch_bounds__(128, KC_BC_MIN_BLOCKS) k_set_bc(DevState s, DevScalars* sc,
+                                                                  const __grid_constant__ BcArgs a) {
+  const unsigned b = blockIdx.x;
+  const int part = b < a.b1 ? 0 : b < a.b2 ? 1 : b < a.b3 ? 2 : 3;
+  const long t = (long)(b - (part == 0 ? 0u : part == 1 ? a.b1 : part == 2 ? a.b2 : a.b3)) * blockDim.x + threadIdx.x;
+  GhostTask g;
+  if (part < 3) face_task(s.gr, part, t, g);
+  else corner_task(s.gr, a.bc, t, g);
+  if (g.n == 0) return;
+  double pp[NV], uu[NV];
+  KC_ROLLED
+  for (int k = 0; k < g.n; ++k) {
+    double q[NV];
+    const long ix = k ? g.x[1][0] : g.x[0][0], iy = k ? g.x[1][1] : g.x[0][1], iz = k ? g.x[1][2] : g.x[0][2];
+    const int e = ghost_prims(s, ix, iy, iz, k ? g.face[1] : g.face[0], a.bc, q);
+    if (e) {
+      set_err(sc, e, cidx(s.gr, ix, iy, iz));
+      return;
+    }
+    for (int iv = 0; iv < NV; ++iv) pp[iv] = k ? 0.5 * (pp[iv] + q[iv]) : q[iv];
+  }
+  Geom geo;
+  geom_cell(s, g.d[0], g.d[1], g.d[2], geo);
+  p2u(pp, uu, geo, a.gam);
+  const long c = cidx(s.gr, g.d[0], g.d[1], g.d[2]);
+  store_cell(s.p, s.gr.nc, c, pp);
+  store_cell(s.u, s.gr.nc, c, uu);
 }
 
 // ---- polar axis overwrite (koral/sim/polaraxis.zig:124) -----------------------
