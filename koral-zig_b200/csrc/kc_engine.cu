@@ -16,6 +16,7 @@
 
 #include <cub/device/device_radix_sort.cuh>
 
+#include "kc_host_copy.cuh"
 #include "kc_kernels.cuh"
 #include "kc_fold.cuh"
 #include "kc_init_lean.cuh"
@@ -862,6 +863,7 @@ int kc_create(const kc_grid* grid, const kc_options* opt, kc_handle** out) {
   *out = nullptr;
   const char* why = validate_config(*grid, *opt);
   kc_handle* h = new kc_handle();
+  hostcopy::handle_made();
   if (why) {
     fail(h, KC_ERR_INVALID_CONFIG, why);
     *out = h;
@@ -977,13 +979,14 @@ void kc_destroy(kc_handle* h) {
   for (void* p : h->allocs) cudaFree(p);
   for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
   if (h->stream) cudaStreamDestroy(h->stream);
+  hostcopy::handle_gone();
   delete h;
 }
 
 static int upload_field(kc_handle* h, double* dst, const double* host, int nv) {
   if (!h || !host) return KC_ERR_INVALID_CONFIG;
   long n = (long)nv * h->gr.nc;
-  int st = cuda_check(h, cudaMemcpyAsync(h->staging, host, n * 8, cudaMemcpyHostToDevice, h->stream), "upload");
+  int st = cuda_check(h, hostcopy::to_device(h->staging, host, n * 8, h->stream), "upload");
   if (st) return st;
   k_aos_to_soa<<<nblk(n, 256), 256, 0, h->stream>>>(h->staging, dst, h->gr.nc, nv);
   return cuda_check(h, cudaStreamSynchronize(h->stream), "upload");
@@ -992,9 +995,7 @@ static int download_field(kc_handle* h, const double* src, double* host, int nv)
   if (!h || !host) return KC_ERR_INVALID_CONFIG;
   long n = (long)nv * h->gr.nc;
   k_soa_to_aos<<<nblk(n, 256), 256, 0, h->stream>>>(src, h->staging, h->gr.nc, nv);
-  int st = cuda_check(h, cudaMemcpyAsync(host, h->staging, n * 8, cudaMemcpyDeviceToHost, h->stream), "download");
-  if (st) return st;
-  return cuda_check(h, cudaStreamSynchronize(h->stream), "download");
+  return cuda_check(h, hostcopy::to_host(host, h->staging, n * 8, h->stream), "download");
 }
 
 int kc_upload_prims(kc_handle* h, const double* p) { return upload_field(h, h->ds.p, p, NV); }
@@ -1004,7 +1005,7 @@ int kc_download_cons(kc_handle* h, double* u) { return download_field(h, h->ds.u
 int kc_upload_flags(kc_handle* h, const int32_t* f) {
   if (!h || !f) return KC_ERR_INVALID_CONFIG;
   long n = 6L * h->gr.nc;
-  int st = cuda_check(h, cudaMemcpyAsync(h->flag_staging, f, n * 4, cudaMemcpyHostToDevice, h->stream), "upload");
+  int st = cuda_check(h, hostcopy::to_device(h->flag_staging, f, n * 4, h->stream), "upload");
   if (st) return st;
   k_flags_to_soa<<<nblk(n, 256), 256, 0, h->stream>>>(h->flag_staging, h->ds.flags, h->gr.nc);
   return cuda_check(h, cudaStreamSynchronize(h->stream), "upload");
@@ -1013,9 +1014,7 @@ int kc_download_flags(kc_handle* h, int32_t* f) {
   if (!h || !f) return KC_ERR_INVALID_CONFIG;
   long n = 6L * h->gr.nc;
   k_flags_to_aos<<<nblk(n, 256), 256, 0, h->stream>>>(h->ds.flags, h->flag_staging, h->gr.nc);
-  int st = cuda_check(h, cudaMemcpyAsync(f, h->flag_staging, n * 4, cudaMemcpyDeviceToHost, h->stream), "download");
-  if (st) return st;
-  return cuda_check(h, cudaStreamSynchronize(h->stream), "download");
+  return cuda_check(h, hostcopy::to_host(f, h->flag_staging, n * 4, h->stream), "download");
 }
 
 int kc_set_counters(kc_handle* h, const kc_counters* c) {
