@@ -554,16 +554,19 @@ void launch_flux_ct(kc_handle* h) {
   else k_ct_rebuild<double><<<nblk(n, 256), 256, 0, h->stream>>>(h->ds);
 }
 
+void launch_update(kc_handle* h, int dt_slot) {
+  PassScope ps(h, KC_PASS_UPDATE);
+  const unsigned nb = nblk((long)h->gr.nx * h->gr.ny * h->gr.nz);
+  h->n_launch += 2;
+  k_update_flux<<<dim3(nb, NV), TPB, 0, h->stream>>>(h->ds, dt_slot);
+  k_update_source<<<nb, TPB, 0, h->stream>>>(h->ds, h->sp.gam, dt_slot);
+}
+
 void launch_op_explicit(kc_handle* h, int dt_slot) {
   launch_wavespeeds(h);
   launch_face_fluxes(h);
   launch_flux_ct(h);
-  const DGrid& gr = h->gr;
-  {
-    PassScope ps(h, KC_PASS_UPDATE);
-    ++h->n_launch;
-    k_update<<<nblk((long)gr.nx * gr.ny * gr.nz), TPB, 0, h->stream>>>(h->ds, h->sp.gam, dt_slot);
-  }
+  launch_update(h, dt_slot);
   launch_calc_u2p(h);
 }
 
@@ -609,12 +612,12 @@ void copy_field(kc_handle* h, double* dst, const double* src) {
   PassScope ps(h, KC_PASS_STAGE);
   cudaMemcpyAsync(dst, src, (size_t)NV * h->gr.nc * 8, cudaMemcpyDeviceToDevice, h->stream);
 }
-// the stage kernels: one thread per domain cell
+// the stage kernels: one thread per domain cell and component
 template <class... A, class... B>
 void launch_stage(kc_handle* h, void (*kernel)(DevState, A...), B... args) {
   PassScope ps(h, KC_PASS_STAGE);
   ++h->n_launch;
-  kernel<<<nblk((long)h->gr.nx * h->gr.ny * h->gr.nz, 256), 256, 0, h->stream>>>(h->ds, args...);
+  kernel<<<dim3(nblk((long)h->gr.nx * h->gr.ny * h->gr.nz, 256), NV), 256, 0, h->stream>>>(h->ds, args...);
 }
 
 // Coefficient slots of a step (run_step fills 0-3 before its first launch)
@@ -1268,12 +1271,7 @@ int kc_debug_phase(kc_handle* h, int phase, double dt) {
     case 0: launch_wavespeeds(h); break;
     case 1: launch_face_fluxes(h); break;
     case 2: launch_flux_ct(h); break;
-    case 3: {
-      const DGrid& gr = h->gr;
-      ++h->n_launch;
-      k_update<<<nblk((long)gr.nx * gr.ny * gr.nz), TPB, 0, h->stream>>>(h->ds, h->sp.gam, coef_slot(h, dt));
-      break;
-    }
+    case 3: launch_update(h, coef_slot(h, dt)); break;
     case 4: launch_calc_u2p(h); break;
     case 5: launch_implicit(h, coef_slot(h, dt)); break;
     case 6: launch_rijvisc(h, coef_slot(h, dt)); break;

@@ -16,7 +16,7 @@
 //                  the bounds; any other chunk (the first, the few that cross a
 //                  binade, a non-finite term) it adds term by term.
 // Measured: the wedge's sums 16 ms to 0.5 ms a row of diagnostics, the 384x360
-// grid's 0.86 to about 0.2 ms.
+// grid's 0.86 to about 0.3 ms.
 #pragma once
 #include <math.h>
 

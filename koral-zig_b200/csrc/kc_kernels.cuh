@@ -49,13 +49,13 @@ struct Range {
   long x0, y0, z0, nx, ny, nz;
 };
 __device__ __forceinline__ bool range_cell(const Range& r, long& ix, long& iy, long& iz) {
-  long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  long n = r.nx * r.ny * r.nz;
-  if (t >= n) return false;
-  ix = r.x0 + t % r.nx;
-  long q = t / r.nx;
-  iy = r.y0 + q % r.ny;
-  iz = r.z0 + q / r.ny;
+  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= r.nx * r.ny * r.nz) return false;
+  // 32-bit divisions: 2^32 cells' fields alone would be 4 TB
+  const unsigned k = (unsigned)t, nx = (unsigned)r.nx, ny = (unsigned)r.ny, q = k / nx, z = q / ny;
+  ix = r.x0 + (k - q * nx);
+  iy = r.y0 + (q - z * ny);
+  iz = r.z0 + z;
   return true;
 }
 
@@ -209,63 +209,57 @@ __global__ void k_flags_to_aos(const int* __restrict__ soa, int* __restrict__ ao
 }
 
 // ---- stage arithmetic (koral/sim.zig:1586-1709) ------------------------------
-// Streaming passes over 13 components, bound by HBM (5.9 TB/s): the derivatives,
+// Streaming passes over 13 components, bound by HBM: the derivatives,
 // combinations and copies that follow each other are one pass each, 19 component
-// reads and writes a step less than one by one, and seven launches.
+// reads and writes a step less than one by one, and seven launches. One thread
+// per cell and component (blockIdx.y): with a cell's 13 in one thread the mid
+// pass took 286 us at 192x180x64 and 9.3 at 32x30, so 255 (6.3 TB/s) and 2.5.
 
 // dst = (1/delta) u + (-1/delta) b over the domain, and the copy ut = u
-__global__ void k_stage_deriv_copy(DevState s, double* dst, const double* b, int delta_slot, double* ut) {
+__global__ void k_stage_deriv_copy(DevState s, double* __restrict__ dst, const double* __restrict__ b, int delta_slot,
+                                   double* __restrict__ ut) {
   const double delta = s.coef[delta_slot];
   Range r = {0, 0, 0, s.gr.nx, s.gr.ny, s.gr.nz};
   long ix, iy, iz;
   if (!range_cell(r, ix, iy, iz)) return;
-  const long c = cidx(s.gr, ix, iy, iz), nc = s.gr.nc;
+  const long k = blockIdx.y * s.gr.nc + cidx(s.gr, ix, iy, iz);
   const double f1 = 1.0 / delta, f2 = -1.0 / delta;
-#pragma unroll
-  for (int iv = 0; iv < NV; ++iv) {
-    const double u = s.u[iv * nc + c];
-    dst[iv * nc + c] = f1 * u + f2 * b[iv * nc + c];
-    ut[iv * nc + c] = u;
-  }
+  const double u = s.u[k];
+  dst[k] = f1 * u + f2 * b[k];
+  ut[k] = u;
 }
 // The end of the first stage: dut1 = (u - ut1) / dt, then u and its copy uforget
 // = ut0 + dt dut1 + fc drt1, and the entropy flags' copy (C copy_entropycount)
-__global__ void k_stage_mid(DevState s, double* dut1, const double* ut1, const double* ut0, const double* drt1,
-                            int dt_slot, int fc_slot, double* uforget) {
+__global__ void k_stage_mid(DevState s, double* __restrict__ dut1, const double* __restrict__ ut1,
+                            const double* __restrict__ ut0, const double* __restrict__ drt1, int dt_slot, int fc_slot,
+                            double* __restrict__ uforget) {
   const double dt = s.coef[dt_slot], fc = s.coef[fc_slot];
   Range r = {0, 0, 0, s.gr.nx, s.gr.ny, s.gr.nz};
   long ix, iy, iz;
   if (!range_cell(r, ix, iy, iz)) return;
-  const long c = cidx(s.gr, ix, iy, iz), nc = s.gr.nc;
+  const long c = cidx(s.gr, ix, iy, iz), nc = s.gr.nc, k = blockIdx.y * nc + c;
   const double f1 = 1.0 / dt, f2 = -1.0 / dt;
-#pragma unroll
-  for (int iv = 0; iv < NV; ++iv) {
-    const long k = iv * nc + c;
-    const double d = f1 * s.u[k] + f2 * ut1[k];
-    const double u = ut0[k] + dt * d + fc * drt1[k];
-    dut1[k] = d;
-    s.u[k] = u;
-    uforget[k] = u;
-  }
-  s.flags[2 * nc + c] = s.flags[0 * nc + c];
+  const double d = f1 * s.u[k] + f2 * ut1[k];
+  const double u = ut0[k] + dt * d + fc * drt1[k];
+  dut1[k] = d;
+  s.u[k] = u;
+  uforget[k] = u;
+  if (blockIdx.y == 0) s.flags[2 * nc + c] = s.flags[0 * nc + c];
 }
 // The end of the step: dut2 = (u - ut2) / dt, u = ut0 + h dut1 + h dut2, then
 // u = u + h drt1 + h drt2
-__global__ void k_stage_end(DevState s, const double* ut2, const double* ut0, const double* dut1, const double* drt1,
-                            const double* drt2, int dt_slot, int h_slot) {
+__global__ void k_stage_end(DevState s, const double* __restrict__ ut2, const double* __restrict__ ut0,
+                            const double* __restrict__ dut1, const double* __restrict__ drt1,
+                            const double* __restrict__ drt2, int dt_slot, int h_slot) {
   const double dt = s.coef[dt_slot], h = s.coef[h_slot];
   Range r = {0, 0, 0, s.gr.nx, s.gr.ny, s.gr.nz};
   long ix, iy, iz;
   if (!range_cell(r, ix, iy, iz)) return;
-  const long c = cidx(s.gr, ix, iy, iz), nc = s.gr.nc;
+  const long k = blockIdx.y * s.gr.nc + cidx(s.gr, ix, iy, iz);
   const double f1 = 1.0 / dt, f2 = -1.0 / dt;
-#pragma unroll
-  for (int iv = 0; iv < NV; ++iv) {
-    const long k = iv * nc + c;
-    const double d = f1 * s.u[k] + f2 * ut2[k];
-    const double u = ut0[k] + h * dut1[k] + h * d;
-    s.u[k] = u + h * drt1[k] + h * drt2[k];
-  }
+  const double d = f1 * s.u[k] + f2 * ut2[k];
+  const double u = ut0[k] + h * dut1[k] + h * d;
+  s.u[k] = u + h * drt1[k] + h * drt2[k];
 }
 // C update_entropy (koral/sim.zig:1683)
 __global__ void __launch_bounds__(128) k_update_entropy(DevState s, double gam) {
@@ -1119,45 +1113,69 @@ __global__ void k_ct_rebuild(DevState s) {
 }
 
 // ---- conserved update + metric source (sim.zig:1140,1542) --------------------
-// 4 resident blocks (128 registers, small spills): measured 4% faster than 168
-__global__ void __launch_bounds__(128, 4) k_update(DevState s, double gam, int dt_slot) {
+// Two streaming kernels bound by HBM: u + du of the flux differences, then
+// + dt times the metric source, the reference's two additions in their order.
+// As one kernel the source's 81 loads and two stress tensors left the registers
+// for too few loads in flight: 924 us at 192x180x64, 19 at 32x30, against 717
+// and 9 of the two.
+
+// u += du, one thread per cell and component (blockIdx.y): with a cell's 13 in
+// one thread 498 us at 192x180x64 and 16 at 32x30, so 379 and 2.7. What is left
+// is the three FP64 divisions per value, more than the 1.15 GB (180 us).
+__global__ void __launch_bounds__(128) k_update_flux(DevState s, int dt_slot) {
   Range r = {0, 0, 0, s.gr.nx, s.gr.ny, s.gr.nz};
   long ix, iy, iz;
   if (!range_cell(r, ix, iy, iz)) return;
-  long nc = s.gr.nc, c = cidx(s.gr, ix, iy, iz);
+  const int iv = blockIdx.y;
   const Grid& g = s.gr.g;
+  const double dx = cell_size(g, ix, 0), dy = cell_size(g, iy, 1), dz = cell_size(g, iz, 2);
+  const double dt = s.coef[dt_slot];
+  const long f0 = iv * s.nf[0] + face_index(s.gr, 0, ix, iy, iz), f1 = iv * s.nf[1] + face_index(s.gr, 1, ix, iy, iz);
+  const long f2 = iv * s.nf[2] + face_index(s.gr, 2, ix, iy, iz);
+  // a collapsed direction's fluxes are never written: zeros
+  const double d0 = s.gr.nx > 1 ? s.flb[0][f0 + 1] - s.flb[0][f0] : 0.0;
+  const double d1 = s.gr.ny > 1 ? s.flb[1][f1 + s.gr.sx] - s.flb[1][f1] : 0.0;
+  const double d2 = s.gr.nz > 1 ? s.flb[2][f2 + s.gr.sx * s.gr.sy] - s.flb[2][f2] : 0.0;
+  const double du = -d0 * dt / dx - d1 * dt / dy - d2 * dt / dz;
+  double* u = s.u + iv * s.gr.nc + cidx(s.gr, ix, iy, iz);
+  double x = *u + du;
+  const bool source = (iv >= UU && iv <= VZ) || iv >= EE;
+  if (!source) x += 0.0 * dt;  // the other components' source
+  *u = x;
+}
+// 4 resident blocks (128 registers, small spills): faster than 168 registers
+__global__ void __launch_bounds__(128, 4) k_update_source(DevState s, double gam, int dt_slot) {
+  Range r = {0, 0, 0, s.gr.nx, s.gr.ny, s.gr.nz};
+  long ix, iy, iz;
+  if (!range_cell(r, ix, iy, iz)) return;
+  const long nc = s.gr.nc, c = cidx(s.gr, ix, iy, iz);
   double pp[NV];
   load_cell(s.p, nc, c, pp);
   Geom geo;
   geom_cell(s, ix, iy, iz, geo);
-  double gdetu = geo.gdet;
-  double ss[NV];
-  for (int i = 0; i < NV; ++i) ss[i] = 0.0;
+  const double gdetu = geo.gdet;
+  double ss[8];
+  for (int i = 0; i < 8; ++i) ss[i] = 0.0;
   double tij[4][4], tl[4][4], rup[4][4], rl[4][4];
   calc_tij(pp, geo, gam, tij);
   lower_second(tij, geo, tl);
   calc_rij(pp, geo, rup);
   lower_second(rup, geo, rl);
-  const int rows[4] = {UU, VX, VY, VZ}, rrows[4] = {EE, FX, FY, FZ};
+#pragma unroll
   for (int a = 0; a < 4; ++a)
+#pragma unroll
     for (int l = 0; l < 4; ++l)
+#pragma unroll
       for (int nu = 0; nu < 4; ++nu) {
-        double k = s.kr[(long)(l * 10 + sym10(nu, a)) * nc + c];
-        ss[rows[nu]] += gdetu * tl[a][l] * k;
-        ss[rrows[nu]] += gdetu * rl[a][l] * k;
+        const double k = s.kr[(long)(l * 10 + sym10(nu, a)) * nc + c];
+        ss[nu] += gdetu * tl[a][l] * k;
+        ss[4 + nu] += gdetu * rl[a][l] * k;
       }
-  double dx = cell_size(g, ix, 0), dy = cell_size(g, iy, 1), dz = cell_size(g, iz, 2);
-  double dt = s.coef[dt_slot];
-  long fx0 = face_index(s.gr, 0, ix, iy, iz), fx1 = face_index(s.gr, 0, ix + 1, iy, iz);
-  long fy0 = face_index(s.gr, 1, ix, iy, iz), fy1 = face_index(s.gr, 1, ix, iy + 1, iz);
-  long fz0 = face_index(s.gr, 2, ix, iy, iz), fz1 = face_index(s.gr, 2, ix, iy, iz + 1);
-  for (int iv = 0; iv < NV; ++iv) {
-    double flxl = s.flb[0][iv * s.nf[0] + fx0], flxr = s.flb[0][iv * s.nf[0] + fx1];
-    double flyl = s.flb[1][iv * s.nf[1] + fy0], flyr = s.flb[1][iv * s.nf[1] + fy1];
-    double flzl = s.flb[2][iv * s.nf[2] + fz0], flzr = s.flb[2][iv * s.nf[2] + fz1];
-    double du = -(flxr - flxl) * dt / dx - (flyr - flyl) * dt / dy - (flzr - flzl) * dt / dz;
-    double uo = s.u[iv * nc + c];
-    s.u[iv * nc + c] = uo + du + ss[iv] * dt;
+  const double dt = s.coef[dt_slot];
+#pragma unroll
+  for (int nu = 0; nu < 4; ++nu) {
+    s.u[(UU + nu) * nc + c] += ss[nu] * dt;
+    s.u[(EE + nu) * nc + c] += ss[4 + nu] * dt;
   }
 }
 
@@ -1184,7 +1202,7 @@ struct ImplExtra {
 };
 // Whether the no-bisection start (the cell's pre-solve state) would have to
 // iterate: its first-rung residual against the Newton core's first exit
-// (conv), as solve_implicit_lab_from evaluates it. Out of line, so that its
+// (conv), as k_implicit_pick evaluates it. Out of line, so that its
 // locals do not enlarge the solve's call frame.
 __device__ __noinline__ bool presolve_needs_newton(const double pp00[NV], const Geom& g, double dt, const ImplArgs& a) {
   double uu00[NV], pc[NV];

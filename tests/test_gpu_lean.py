@@ -39,10 +39,11 @@ def test_init_columns_with_spin(spin):
     _same(gpu, orc)
 
 
-@pytest.mark.parametrize("shape", [(31, 21, 1), (37, 33, 1), (148, 9, 1), (149, 33, 4)])
+@pytest.mark.parametrize("shape", [(31, 21, 1), (37, 33, 1), (148, 9, 1), (149, 33, 4), (11, 13, 7)])
 def test_steps_at_the_edges_of_the_solve_launches(shape):
-    """651 and 1221 cells (2 and 3 cells a warp), few theta rows, and 19668
-    cells (full warps, the last one partly filled)."""
+    """651 and 1221 cells (2 and 3 cells a warp), few theta rows, 19668 cells
+    (full warps, the last one partly filled), and a small grid with faces in
+    all three directions (the update's streaming passes by component)."""
     gpu, orc = _pair(*shape)
     for _ in range(2):
         gpu.step()
