@@ -303,64 +303,29 @@ KC_HD void lag_opac(RadState& st, const RadState& st00) {
   st.opac.rad_ross = st00.opac.rad_ross;
 }
 
-// The loop state of the Newton core at the top of an iteration: what a paused
-// solve (RESUME) carries to its next call. iter = iterations done, 0 = not started.
-struct CoreCarry {
-  double uu[NV], pp[NV];
-  RadState state;
-  int fret, iter;
-};
 // C solve_implicit_lab_4dprim Newton core (implicit.zig:642). Returns 1 on
 // success (pp_out written, *iters set), 0 on failure.
-// RESUME = false is the reference's core as is. RESUME = true starts from
-// *carry when carry->iter > 0, runs at most `budget` iterations and then, if the
-// solve has not ended, saves its loop state to *carry and returns 2; the
-// iterations run are those of the uninterrupted core, so a solve split over
-// several calls ends exactly as it would in one.
-template <bool RESUME>
-KC_HDN int solve_4dprim_core_t(const double uu00[NV], const RadState& state00, const double pp0in[NV], const Geom& g,
-                               double dt, double gam, const RadParams& rad, const OpacParams& op, double opdamp,
-                               const ImplicitParams& ip, int whichprim, int whicheq, int whichframe, double pp_out[NV],
-                               int* iters_out, CoreCarry* carry, int budget) {
+KC_HDN int solve_4dprim_core(const double uu00[NV], const RadState& state00, const double pp0in[NV], const Geom& g,
+                             double dt, double gam, const RadParams& rad, const OpacParams& op, double opdamp,
+                             const ImplicitParams& ip, int whichprim, int whicheq, int whichframe, double pp_out[NV],
+                             int* iters_out) {
   double uu[NV], pp[NV];
   int sh = (whichprim == PRIM_MHD) ? UU : EE;
   double conv = (whicheq == EQ_ENTROPY) ? ip.entrconv : ip.conv;
   bool slim = whicheq != EQ_ENTROPY;
-  int fret, iter;
-  RadState state;
-  if (RESUME && carry->iter > 0) {
-    for (int i = 0; i < NV; ++i) {
-      uu[i] = carry->uu[i];
-      pp[i] = carry->pp[i];
-    }
-    state = carry->state;
-    fret = carry->fret;
-    iter = carry->iter;
-  } else {
-    for (int i = 0; i < NV; ++i) {
-      uu[i] = uu00[i];
-      pp[i] = pp0in[i];
-    }
-    fret = apply_constraints(pp, uu, uu00, g, gam, rad, ip, whichprim);
-    fill_rad_state(pp, g, gam, op, !slim, state);
-    if (ip.lag_opac) lag_opac(state, state00);
-    iter = 0;
+  for (int i = 0; i < NV; ++i) {
+    uu[i] = uu00[i];
+    pp[i] = pp0in[i];
   }
-  const int stop = RESUME ? iter + budget : 0;
+  int fret = apply_constraints(pp, uu, uu00, g, gam, rad, ip, whichprim);
+  RadState state;
+  fill_rad_state(pp, g, gam, op, !slim, state);
+  if (ip.lag_opac) lag_opac(state, state00);
+  int iter = 0;
   double f1[4], f2[4], jac[4][4];
   bool failed = false;
   bool success = false;
   while (true) {
-    if (RESUME && iter >= stop) {
-      for (int i = 0; i < NV; ++i) {
-        carry->uu[i] = uu[i];
-        carry->pp[i] = pp[i];
-      }
-      carry->state = state;
-      carry->fret = fret;
-      carry->iter = iter;
-      return 2;
-    }
     iter += 1;
     double ppp[NV];
     for (int i = 0; i < NV; ++i) ppp[i] = pp[i];
@@ -474,15 +439,6 @@ KC_HDN int solve_4dprim_core_t(const double uu00[NV], const RadState& state00, c
   for (int i = 0; i < NV; ++i) pp_out[i] = pp[i];
   *iters_out = iter;
   return 1;
-}
-// the reference's core (koral/solve/implicit.zig:642): 1 on success (pp_out,
-// *iters_out written), 0 on failure
-KC_HD int solve_4dprim_core(const double uu00[NV], const RadState& state00, const double pp0in[NV], const Geom& g,
-                            double dt, double gam, const RadParams& rad, const OpacParams& op, double opdamp,
-                            const ImplicitParams& ip, int whichprim, int whicheq, int whichframe, double pp_out[NV],
-                            int* iters_out) {
-  return solve_4dprim_core_t<false>(uu00, state00, pp0in, g, dt, gam, rad, op, opdamp, ip, whichprim, whicheq,
-                                    whichframe, pp_out, iters_out, nullptr, 0);
 }
 
 // The per-solve preamble of C solve_implicit_lab (implicit.zig:927-961): the
@@ -601,59 +557,6 @@ KC_HDN int implicit_first_exit(double uu[NV], double pp[NV], const Geom& g, doub
   for (int i = 0; i < NV; ++i) pp[i] = pc[i];
   p2u(pc, uu, g, gam);
   return 1;
-}
-
-// The same ladder started from a learned state in place of the bisection warm
-// start (the learned-guess form; it has no counterpart in the reference).
-// The start fluid is decided as solve_implicit_lab decides it. A cell the
-// pre-solve state already satisfies (first-rung residual below conv, the
-// core's first exit) is finished there, as the core would finish it, so a
-// prediction error never costs such a cell an iteration; the others run the
-// ladder from whichever of the pre-solve and the learned state has the
-// smaller first-rung residual (starting every such cell from the learned
-// state measured slower: the prediction is worse than the pre-solve state for
-// a part of them).
-// The learned start's preamble: the reference conserveds and state of the
-// pre-solve primitives, the start fluid, and the core's first exit on rung 0
-// (lab frame, energy equation) at the pre-solve state; returns 1 when that exit
-// is taken (uu, pp written), else 0 with pre.pp0 the one of the pre-solve and
-// the learned state that has the smaller rung-0 first residual.
-KC_HDN int implicit_prepare_from(double uu[NV], double pp[NV], const Geom& g, double dt, double gam,
-                                 const RadParams& rad, const OpacParams& op, const ImplicitParams& ip,
-                                 const double guess[NV], ImplicitPre& pre) {
-  p2u(pp, pre.uu00, g, gam);
-  double ehat = -calc_ff_rtt(pp, g, nullptr);
-  fill_rad_state(pp, g, gam, op, true, pre.state00);
-  pre.startwith = (ehat < ip.threshold * pp[UU]) ? PRIM_RAD : PRIM_MHD;
-  double pc[NV];
-  double e0 = implicit_start_residual(pre.uu00, pre.state00, pp, g, dt, gam, rad, op, 1.0, ip, pre.startwith, pc);
-  if (e0 < ip.conv) {
-    for (int i = 0; i < NV; ++i) pp[i] = pc[i];
-    p2u(pc, uu, g, gam);
-    return 1;
-  }
-  double e1 = implicit_start_residual(pre.uu00, pre.state00, guess, g, dt, gam, rad, op, 1.0, ip, pre.startwith, pc);
-  bool learned = e1 < e0;
-  for (int i = 0; i < NV; ++i) pre.pp0[i] = learned ? guess[i] : pp[i];
-  return 0;
-}
-// the result of the core's first exit on rung 0
-KC_HD ImplicitResult implicit_first_exit_result(int startwith) {
-  ImplicitResult res;
-  res.ok = 1;
-  res.rung = 0;
-  res.iters = 1;
-  res.whichprim = startwith;
-  res.whicheq = EQ_ENERGY;
-  res.whichframe = FRAME_LAB;
-  return res;
-}
-KC_HDN ImplicitResult solve_implicit_lab_from(double uu[NV], double pp[NV], const Geom& g, double dt, double gam,
-                                              const RadParams& rad, const OpacParams& op, const ImplicitParams& ip,
-                                              const double guess[NV]) {
-  ImplicitPre pre;
-  if (implicit_prepare_from(uu, pp, g, dt, gam, rad, op, ip, guess, pre)) return implicit_first_exit_result(pre.startwith);
-  return implicit_ladder(uu, pp, g, dt, gam, rad, op, ip, pre);
 }
 
 }  // namespace kp

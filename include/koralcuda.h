@@ -61,17 +61,15 @@ enum { KC_PLAIN_FP64 = 0, KC_MIXED = 1 };
 enum { KC_FP32_PPM = 2, KC_FP32_LAXF = 4, KC_FP32_CT = 8, KC_FP32_FLUX = 16 };
 enum { KC_GUESS_PLAIN = 0, KC_GUESS_MLP = 1 };
 /* implicit pass forms (no reference counterpart; all bit-identical to the
- * reference's per-cell solveImplicitLab loop, koral/sim.zig:1715):
- * PER_CELL one thread per cell; COMPACTING a persistent lane-refilling state
- * machine; SPLIT an opening kernel that finishes every cell passing the Newton
- * core's first residual test at its warm start and a ladder kernel over the
- * compacted rest; SORTED (the batch entry points only) the per-cell kernel over
- * the cells sorted by start fluid, optical depth and temperature; RUNGS (the
- * batch entry points only) the sorted cells prepared once (warm start and
- * reference state), then one launch per rung of the ladder over the cells the
- * earlier rungs left unsolved, compacted between rungs; ITERS (the batch entry
- * points only) as RUNGS, with every rung run in launches of at most 8 Newton
- * iterations per cell, the cells still iterating compacted between launches */
+ * reference's per-cell solveImplicitLab loop, koral/sim.zig:1715).
+ * In a step: PER_CELL a warm-start kernel and a ladder kernel, one thread per
+ * cell; COMPACTING a persistent lane-refilling state machine; SPLIT an opening
+ * kernel that finishes every cell passing the Newton core's first residual test
+ * at its warm start and a ladder kernel over the compacted rest.
+ * In the batch entry points: PER_CELL one kernel, each thread its own cells, no
+ * scratch; COMPACTING a warm-start kernel and a persistent solve whose lanes take
+ * the next cell when theirs ends; SORTED, RUNGS and ITERS the same over the cells
+ * sorted by start fluid, optical depth and temperature. */
 enum {
   KC_IMPLICIT_PER_CELL = 0,
   KC_IMPLICIT_COMPACTING = 1,
@@ -272,11 +270,12 @@ int kc_set_graph(kc_handle* h, int32_t on);
  * once into shared memory, 2 the same with the PPM stencil rows staged in
  * shared memory too. kc_autotune picks among them. */
 int kc_set_face_tiles(kc_handle* h, int32_t mode);
-/* Threads per block of the per-cell implicit kernel (no reference counterpart;
- * every size gives the same bits): one block fills an SM, so the size sets the
- * register budget: 256 (255 registers per thread, 8 warps), 384 (168, 12 warps;
- * the default) or 512 (128, 16 warps). Other sizes: KC_ERR_INVALID_CONFIG.
- * kc_autotune picks among them. */
+/* Threads per block of the per-cell form's ladder kernel (no reference
+ * counterpart; every size gives the same bits): one block fills an SM, so the
+ * size sets the register budget: 256 (255 registers per thread, 8 warps), 384
+ * (168, 12 warps; the default) or 512 (128, 16 warps). Other sizes:
+ * KC_ERR_INVALID_CONFIG. A grid of fewer than 8 warps an SM runs small blocks of
+ * the 255-register kernel whatever the size. kc_autotune picks among them. */
 int kc_set_implicit_threads(kc_handle* h, int32_t threads);
 
 /* The autotuner's choice (no reference counterpart): implicit form

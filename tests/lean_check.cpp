@@ -219,7 +219,7 @@ int main(int argc, char** argv) {
       if (k == 3) u2[RHO] = -u2[RHO];
       memcpy(p2, p1, sizeof p2);
       const int et = k == 1 ? ETYPE_ENTROPY : ETYPE_HOT;
-      const int ra = u2p_solver_w_inl(u2, p1, g, et, gam), rb = kc::lean::u2p_w(u2, p2, g, et, gam, true);
+      const int ra = u2p_solver_w(u2, p1, g, et, gam), rb = kc::lean::u2p_w(u2, p2, g, et, gam, true);
       if (ra != rb || !same(p1, p2, NV)) ++bad_w;
     }
   }
