@@ -370,7 +370,7 @@ def run_implicit(args, rank, world, local):
                    "rungs": np.bincount(res[ok, 1], minlength=6).tolist()},
         "e2e": {"value": n * ke / te, "unit": IMPL_UNIT, "h2d_bytes_per_step": n * (23 + 1 + 13) * 8,
                 "d2h_bytes_per_step": n * (13 * 8 + 24), "steps": ke, "timer": "host wall clock (synchronous API)"},
-        "roofline": {"bound": "hbm", "kernel": "k_implicit_batch", "achieved": achieved, "peak": peaks["hbm_gbs"],
+        "roofline": {"bound": "hbm", "kernel": "k_batch_solve", "achieved": achieved, "peak": peaks["hbm_gbs"],
                      "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"], "traffic": None,
                      "algorithmic_bytes": bpc * n},
         "clocks": clk, "gpu_launches": args.steps * batch_launches(IMPLICIT_MODES[args.implicit_mode]),
