@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 
 
 @pytest.fixture(scope="module")
-def checker(tmp_path_factory):
+def lean_binary(tmp_path_factory):
     exe = tmp_path_factory.mktemp("lean") / "lean_check"
     subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-Wno-unknown-pragmas", "-o", str(exe),
                     os.path.join(HERE, "lean_check.cpp")], check=True)
@@ -49,26 +49,26 @@ def cells(tmp_path_factory):
 
 
 @pytest.mark.parametrize("variant", range(12))
-def test_lean_solve_is_bitwise_the_plain_solve(checker, cells, variant):
+def test_lean_solve_is_bitwise_the_plain_solve(lean_binary, cells, variant):
     """Each option that changes the solve's path (lean_check.cpp's variants:
     bisection off, unscaled Jacobian, lagged opacities, no ceiling and no entropy
     fallback, damped levels, opacity channels, another adiabatic index, tight
     convergence), with every rung of the ladder reached."""
     path, n = cells
-    r = subprocess.run([checker, path, str(n), str(variant)], check=True, capture_output=True, text=True)
+    r = subprocess.run([lean_binary, path, str(n), str(variant)], check=True, capture_output=True, text=True)
     bad, bad_w, ok, failed, *rungs = (int(x) for x in r.stdout.split())
     assert bad == 0 and bad_w == 0, r.stderr
     assert ok > 0 and failed > 0 and ok + failed == n and sum(1 for x in rungs if x) >= 3
 
 
 @pytest.mark.parametrize("spin", [0.0, 0.5, -0.3, 0.95])
-def test_torus_functions_are_bitwise_the_plain_ones(checker, spin):
-    r = subprocess.run([checker, "init", str(spin)], check=True, capture_output=True, text=True)
+def test_torus_functions_are_bitwise_the_plain_ones(lean_binary, spin):
+    r = subprocess.run([lean_binary, "init", str(spin)], check=True, capture_output=True, text=True)
     bad, n = (int(x) for x in r.stdout.split())
     assert bad == 0 and n > 100
 
 
-def test_parallel_fold_is_bitwise_the_serial_sum(checker):
-    r = subprocess.run([checker, "fold"], check=True, capture_output=True, text=True)
+def test_parallel_fold_is_bitwise_the_serial_sum(lean_binary):
+    r = subprocess.run([lean_binary, "fold"], check=True, capture_output=True, text=True)
     bad, mapped = (int(x) for x in r.stdout.split())
     assert bad == 0 and mapped > 10000
