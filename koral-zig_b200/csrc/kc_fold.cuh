@@ -56,14 +56,16 @@ KC_HD FoldRun fold_term(double x) {
     r.ok = 0;
     return r;
   }
-  const double f = ::floor(x), fr = x - f;
+  // the midpoint f + 1/2 is exact for every |x| < 2^50; x - f is not (for x just
+  // above -1/2 it rounds to 1/2, which would make a tie of x)
+  const double f = ::floor(x), mid = f + 0.5;
   const long long F = (long long)f;
-  if (fr == 0.5) {
+  if (x == mid) {
     // to the even sum
     r.m.d0 = F + (F & 1);
     r.m.d1 = F + ((F + 1) & 1);
   } else {
-    r.m.d0 = r.m.d1 = F + (fr > 0.5);
+    r.m.d0 = r.m.d1 = F + (x > mid);
   }
   r.lo = F < 0 ? -F : 0;
   r.hi = F >= 0 ? F + 1 : 0;

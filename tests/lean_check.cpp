@@ -80,13 +80,38 @@ static int check_init(double a) {
   return 0;
 }
 
+// One term beside every multiple of half an ulp (the multiple and its neighbours on
+// both sides) added to a sum of either sign and parity, through the term's map and
+// as an addition
+static long check_fold_ties() {
+  using namespace kc;
+  long bad = 0;
+  for (int sign = -1; sign <= 1; sign += 2)
+    for (int e : {-950, -3, 0, 40, 900})
+      for (int odd = 0; odd < 2; ++odd)
+        for (int h = -9; h <= 9; ++h) {
+          const double ulp = ldexp(1.0, e - 52), half = 0.5 * h;
+          const double near[] = {half, nextafter(half, -1e9), nextafter(half, 1e9), nextafter(nextafter(half, -1e9), -1e9),
+                                 nextafter(nextafter(half, 1e9), 1e9)};
+          for (double x : near) {
+            const double v = x * ulp, sum0 = sign * (ldexp(1.5, e) + odd * ulp);
+            double sum = sum0, acc = sum0;
+            sum += v;
+            const long long key = fold_key(sum0);
+            const FoldRun r = fold_term(v * fold_scale(key));
+            const FoldChunk c = {r.m, r.lo, r.hi, r.ok ? key : 0};
+            bad += !fold_apply(acc, c) || !same(&sum, &acc, 1);
+          }
+        }
+  return bad;
+}
 // The ordered fold's maps, chunk by chunk, against the serial sum: sums that grow
 // through binades, of one sign and of both, ties (few-bit terms), zeros, a
 // non-finite term
 static int check_fold() {
   using namespace kc;
   std::mt19937_64 r(3);
-  long bad = 0, mapped = 0;
+  long bad = check_fold_ties(), mapped = 0;
   for (int t = 0; t < 400; ++t) {
     const int kind = t % 8, chunk = 1 << (5 + t % 4);
     std::vector<double> v(2000 + r() % 20000);
