@@ -452,9 +452,10 @@ void launch_implicit(kc_handle* h, int dt_slot) {
   const int lanes = solve_lanes(ndom, h->nsm);
   const long nthread = (ndom + lanes - 1) / lanes * 32;
   h->n_launch += 2;
-  if (x.guess)
-    k_implicit_pick<<<nblk(nthread, KC_PICK_TPB), KC_PICK_TPB, SharedCell::bytes(KC_PICK_TPB), st>>>(h->ds, h->dsc, a, wb,
-                                                                                                    x.guess, lanes);
+  const unsigned np = nblk(nthread, KC_PICK_TPB);
+  const size_t smp = SharedCell::bytes(KC_PICK_TPB);
+  if (x.guess && h->hcap > 0) k_implicit_pick<true><<<np, KC_PICK_TPB, smp, st>>>(h->ds, h->dsc, a, wb, x, lanes);
+  else if (x.guess) k_implicit_pick<false><<<np, KC_PICK_TPB, smp, st>>>(h->ds, h->dsc, a, wb, x, lanes);
   else
     k_implicit_warm<<<nblk(nthread, KC_WARM_TPB), KC_WARM_TPB, 0, st>>>(h->ds, a, wb, lanes);
   // the learned-guess and harvest forms in the default block. A grid of few warps
@@ -897,7 +898,8 @@ int kc_create(const kc_grid* grid, const kc_options* opt, kc_handle** out) {
   if (!st) st = smem((const void*)k_implicit<256>, 256);
   if (!st) st = smem((const void*)k_implicit<384>, 384);
   if (!st) st = smem((const void*)k_implicit<512>, 512);
-  if (!st) st = smem((const void*)k_implicit_pick, KC_PICK_TPB);
+  if (!st) st = smem((const void*)k_implicit_pick<false>, KC_PICK_TPB);
+  if (!st) st = smem((const void*)k_implicit_pick<true>, KC_PICK_TPB);
   if (!st) st = smem((const void*)k_implicit_ext<false>, KC_IMPLICIT_TPB);
   if (!st) st = smem((const void*)k_implicit_ext<true>, KC_IMPLICIT_TPB);
   if (st) return st;

@@ -1433,10 +1433,20 @@ __global__ void __launch_bounds__(NT, 1) k_implicit(const __grid_constant__ DevS
 // residual.
 enum : int { START_FLUID = 3, START_LEARNED = 4, START_DONE = 8 };  // of WarmBuf::startwith
 constexpr int KC_PICK_TPB = 128;
+// one training pair: the pre-solve state pp00 and the solution pp of a solve that
+// started from the fluid sw
+__device__ __forceinline__ void harvest_pair(const ImplExtra& x, const double pp00[NV], const double pp[NV], const Geom& g,
+                                             double dt, int sw) {
+  const unsigned long long k = atomicAdd(x.hcount, 1ULL);
+  if ((long)k >= x.hcap) return;
+  mlp_features_raw(pp00, dt, g.gdet, g.alpha, sw, x.hx + k * MLP_IN);
+  mlp_targets_raw(pp00, pp, sw, x.ht + k * MLP_OUT);
+}
+template <bool HARVEST>
 __global__ void __launch_bounds__(KC_PICK_TPB, 3) k_implicit_pick(const __grid_constant__ DevState s, DevScalars* sc,
                                                                   const __grid_constant__ ImplArgs a,
-                                                                  const __grid_constant__ WarmBuf wb, const double* guess,
-                                                                  int lanes) {
+                                                                  const __grid_constant__ WarmBuf wb,
+                                                                  const __grid_constant__ ImplExtra x, int lanes) {
   extern __shared__ __align__(16) double implicit_smem[];
   const int lane = threadIdx.x & 31;
   const long t = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32 * lanes + lane;
@@ -1480,7 +1490,7 @@ __global__ void __launch_bounds__(KC_PICK_TPB, 3) k_implicit_pick(const __grid_c
   KC_ROLLED
   for (int k = 0; k < 2 && !done; ++k) {
     if (k)
-      for (int i = 0; i < NV; ++i) pp[i] = guess[i * nd + td];
+      for (int i = 0; i < NV; ++i) pp[i] = x.guess[i * nd + td];
     const double e = lean::start_residual(cell, pp, fluid, a.gam, a.rp, a.op, a.ip);
     if (k == 0) e0 = e;
     else learned = e < e0;
@@ -1492,6 +1502,11 @@ __global__ void __launch_bounds__(KC_PICK_TPB, 3) k_implicit_pick(const __grid_c
   double uu[NV];
   const lean::CellGeom q = cell.geom();
   p2u(pp, uu, q.g, a.gam);
+  if (HARVEST && x.hx && !x.hfilter) {  // the filter leaves these cells out
+    double pp00[NV];
+    load_cell(s.p, nc, c, pp00);
+    harvest_pair(x, pp00, pp, q.g, cell.dt_, fluid);
+  }
   s.flags[5 * nc + c] = 0;
   store_cell<true>(s.u, nc, c, uu);
   store_cell<true>(s.p, nc, c, pp);
@@ -1535,14 +1550,8 @@ struct ExtSrc : StepSrc {
       double pp00[NV];
       load_cell(s.p, s.gr.nc, c, pp00);
       const lean::CellGeom g = cell.geom();
-      if (!x.hfilter || presolve_needs_newton(pp00, g.g, cell.dt_, a)) {
-        unsigned long long k = atomicAdd(x.hcount, 1ULL);
-        if ((long)k < x.hcap) {
-          const int sw = wb.startwith[t] & START_FLUID;
-          mlp_features_raw(pp00, cell.dt_, g.g.gdet, g.g.alpha, sw, x.hx + k * MLP_IN);
-          mlp_targets_raw(pp00, q, sw, x.ht + k * MLP_OUT);
-        }
-      }
+      if (!x.hfilter || presolve_needs_newton(pp00, g.g, cell.dt_, a))
+        harvest_pair(x, pp00, q, g.g, cell.dt_, wb.startwith[t] & START_FLUID);
     }
     StepSrc::done(cell, q, r);
   }

@@ -95,3 +95,36 @@ def test_batch_forms_agree(n):
     for mode in (1, 3, 5):
         got = kc.implicit_batch(opt, geom, dt, pp, mode=mode)
         assert np.array_equal(_bits(got[0]), _bits(ref[0])) and np.array_equal(got[1], ref[1])
+
+
+def _pairs(sim, cap=8192):
+    x, t = sim.get_harvest(cap)
+    return {r.tobytes() for r in np.concatenate([x, t], axis=1)}
+
+
+def test_harvest_records_first_exits_under_the_guess():
+    """With a guess installed, the cells whose pre-solve state already passes the
+    first residual test are finished before the ladder; the unfiltered harvest
+    records them all the same, as the run without a bisection does (its pairs less
+    those of its filtered harvest)."""
+    kc = koralcuda()
+    kc.lib()
+    grid = kc.puffy_grid(40, 30, 1)
+    rng = np.random.default_rng(2)
+    w = rng.normal(0.0, 0.05, kc.KC_MLP_NWEIGHTS)
+    w[16:32], w[36:40] = 1.0, 1.0  # the standard deviations
+    got = {}
+    for guess in (False, True):
+        for mode in (0, 1):
+            sim = kc.Sim(grid, kc.puffy_options(radimp_start_with_bisect=0))
+            sim.initPuffy(1e-3, 1e-3, 5)
+            sim.step()
+            dt = 1e-6 * sim.cflDt()  # short enough that some cells need no iteration
+            if guess:
+                sim.set_guess(w)
+            sim.harvest_implicit(8192)
+            sim.set_harvest_filter(mode)
+            sim.debug_phase(5, dt)
+            got[guess, mode] = _pairs(sim)
+    first = got[False, 0] - got[False, 1]
+    assert len(first) > 20 and first <= got[True, 0] and not first & got[True, 1]
