@@ -703,7 +703,9 @@ KC_HD void solve_cells(Src& src, Cell& cell, double gam, const RadParams& rad, c
   const Consts& c = op.c;
   enum { BASE, COLUMN, TRIAL };
   enum { GOING, SOLVED, FAILED };
-  const int nrung = 6 * (ip.opdamp_maxlevels + 1);
+  // none for a negative number of levels; no run reaches the upper bound
+  const int levels = ip.opdamp_maxlevels < 0 ? 0 : ip.opdamp_maxlevels < 1 << 28 ? ip.opdamp_maxlevels + 1 : 1 << 28;
+  const int nrung = 6 * levels;
   double pp[NV], uu[NV];
   Kin kin;
   double ppp[4] = {0, 0, 0, 0}, f1[4] = {0, 0, 0, 0};
@@ -711,6 +713,11 @@ KC_HD void solve_cells(Src& src, Cell& cell, double gam, const RadParams& rad, c
   int stage = BASE, iter = 0, j = 0, rungs = 0, ir = 0, startwith = PRIM_MHD;
   int whicheq = EQ_ENERGY, whichframe = FRAME_LAB;
   bool mhd = true, first = true;  // first: no constraint applied yet in this rung
+  if (nrung == 0) {  // a ladder without rungs fails every cell
+    const ImplicitResult none = {0, -1, 0, PRIM_RAD, EQ_ENERGY, FRAME_LAB};
+    while (src.take(cell, pp, startwith)) src.done(cell, pp, none);
+    return;
+  }
   if (!src.take(cell, pp, startwith)) return;
   mhd = startwith == PRIM_MHD;
   KC_ROLLED
@@ -798,7 +805,7 @@ KC_HD void solve_cells(Src& src, Cell& cell, double gam, const RadParams& rad, c
       // ---- the rung ends: the next one, or the next cell -------------------------------
       if (out == SOLVED && iter > ip.maxiter) out = FAILED;
       rungs += 1;
-      if (out == SOLVED || rungs == nrung) {
+      if (out == SOLVED || rungs >= nrung) {
         ImplicitResult res;
         res.ok = out == SOLVED;
         res.rung = res.ok ? ir : -1;

@@ -174,6 +174,7 @@ int main(int argc, char** argv) {
   if (variant == 7) op.ch.comptonization = 0, op.ch.kleinnishina = 0;
   if (variant == 8) op.ch.synchrotron = 0, op.kappaes_mode = KAPPAES_NONE;
   if (variant == 10) op.ch.bremsstrahlung = 0, ip.maxiter = 20;
+  if (variant >= 12) ip.opdamp_maxlevels = 11 - variant;  // a ladder without rungs
   if (variant == 11) ip.convrelerr = 1.0e-12, ip.convrel = 1.0e-13;  // many iterations
   long bad = 0, bad_w = 0, ok = 0, rungs[7] = {0};
   for (long c = 0; c < n; ++c) {

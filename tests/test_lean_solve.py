@@ -61,6 +61,17 @@ def test_lean_solve_is_bitwise_the_plain_solve(lean_binary, cells, variant):
     assert ok > 0 and failed > 0 and ok + failed == n and sum(1 for x in rungs if x) >= 3
 
 
+@pytest.mark.parametrize("variant", [12, 15])
+def test_ladder_without_rungs_fails_every_cell(lean_binary, cells, variant):
+    """A negative radimp_opdamp_maxlevels leaves the ladder no rung: every cell fails
+    at once with its state untouched, as in the plain solve."""
+    path, n = cells
+    r = subprocess.run([lean_binary, path, str(n), str(variant)], check=True, capture_output=True, text=True, timeout=120)
+    bad, bad_w, ok, failed, *rungs = (int(x) for x in r.stdout.split())
+    assert bad == 0 and bad_w == 0, r.stderr
+    assert ok == 0 and failed == n
+
+
 @pytest.mark.parametrize("spin", [0.0, 0.5, -0.3, 0.95])
 def test_torus_functions_are_bitwise_the_plain_ones(lean_binary, spin):
     r = subprocess.run([lean_binary, "init", str(spin)], check=True, capture_output=True, text=True)
