@@ -2,6 +2,8 @@
 the implicit and u2p passes around the warp's cell counts, the init's columns with
 spin, the ordered folds around the chunk size, the ghost fill on every kind of
 boundary; all bit for bit against the oracle."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -128,3 +130,17 @@ def test_harvest_records_first_exits_under_the_guess():
             got[guess, mode] = _pairs(sim)
     first = got[False, 0] - got[False, 1]
     assert len(first) > 20 and first <= got[True, 0] and not first & got[True, 1]
+
+
+@pytest.mark.parametrize("n", [1, 40000])
+def test_batch_calls_refuse_null_arrays(n):
+    """Each host array of the batch calls, below and above the size from which large
+    arrays are copied by several threads."""
+    kc = koralcuda()
+    lib = kc.lib()
+    opt = kc.puffy_options()
+    arr = [np.zeros((n, 23)), np.zeros((n, 13)), np.zeros((n, 13)), np.zeros((n, 6), np.int32)]
+    for k in range(4):
+        p = [None if i == k else a.ctypes.data for i, a in enumerate(arr)]
+        assert lib.kc_implicit_batch(ctypes.byref(opt), n, *p, 0) == kc.KC_ERR_INVALID_CONFIG
+        assert lib.kc_u2p_batch(ctypes.byref(opt), n, *p) == kc.KC_ERR_INVALID_CONFIG
