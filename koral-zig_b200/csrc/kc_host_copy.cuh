@@ -18,7 +18,6 @@
 
 #include <atomic>
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 namespace kc {
@@ -122,7 +121,7 @@ inline cudaError_t copy(void* dev, const void* host, size_t n, bool up, cudaStre
         for (; nt < kWorkers && nt < cores; ++nt)
           th[nt] = std::thread(work, device, a.mem + nt * kSlots * kChunk, (unsigned char*)dev, (unsigned char*)host, n,
                                up, st, &next, &err);
-      } catch (const std::system_error&) {
+      } catch (...) {  // no thread, or no memory for one
       }
       work(device, a.mem, (unsigned char*)dev, (unsigned char*)host, n, up, st, &next, &err);
       for (int k = 1; k < kWorkers; ++k)
