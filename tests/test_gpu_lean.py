@@ -144,3 +144,46 @@ def test_batch_calls_refuse_null_arrays(n):
         p = [None if i == k else a.ctypes.data for i, a in enumerate(arr)]
         assert lib.kc_implicit_batch(ctypes.byref(opt), n, *p, 0) == kc.KC_ERR_INVALID_CONFIG
         assert lib.kc_u2p_batch(ctypes.byref(opt), n, *p) == kc.KC_ERR_INVALID_CONFIG
+
+
+def _inversion_cells(kc, opt, n):
+    """Seeded cells as inputs of the inversion: rows of primitives as conserveds are
+    states like any other to it, solvable or not."""
+    geom, _, pp = kc.synth_implicit_cells(opt, n, 11)
+    uu = pp * geom[:, 20:21]
+    uu[:, 1] = -uu[:, 0] - uu[:, 1]  # T^t_t
+    uu[:, 9] = -uu[:, 9]
+    return geom, uu, pp
+
+
+def test_small_host_batches_alone_and_at_once():
+    """Host-array calls whose arrays fit the fixed device array (5,188 cells of an
+    inversion do, 5,190 do not), one after the other and from four threads, of which
+    one at a time has it: the rows are those of one large call."""
+    import threading
+
+    kc = koralcuda()
+    kc.lib()
+    opt = kc.puffy_options()
+    geom, uu, pp = _inversion_cells(kc, opt, 6000)
+    ref = kc.u2p_batch(opt, geom, uu, pp)
+    geo2, dt2, pp2 = kc.synth_implicit_cells(opt, 40, 4)
+    ref2 = kc.implicit_batch(opt, geo2, dt2, pp2, mode=5)
+    bad = []
+
+    def calls(sizes):
+        for n in sizes:
+            got = kc.u2p_batch(opt, geom[:n], uu[:n], pp[:n])
+            if not (np.array_equal(_bits(got[0]), _bits(ref[0][:n])) and np.array_equal(got[1], ref[1][:n])):
+                bad.append(n)
+        got = kc.implicit_batch(opt, geo2, dt2, pp2, mode=5)
+        if not (np.array_equal(_bits(got[0]), _bits(ref2[0])) and np.array_equal(got[1], ref2[1])):
+            bad.append("solve")
+
+    calls([1, 5188, 5189, 5190, 33])
+    th = [threading.Thread(target=calls, args=([n, 7 * n, 5188, n, 1] * 4,)) for n in (3, 100, 333, 740)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not bad
