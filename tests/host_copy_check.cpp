@@ -2,6 +2,8 @@
 // it makes. The stand-in's copies are deferred as far as the real ones may be: to
 // the event or stream synchronisation that waits for them, so a slot used again too
 // early, or read too early, shows in the bytes.
+#include <sys/mman.h>
+
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -34,6 +36,13 @@ void run_to(size_t k) {
     memcpy(o.dst, o.src, o.n);
   }
 }
+std::vector<void*> taken;  // memory of the runtime's own
+void device_reset() {      // ends the locking and the runtime's memory
+  std::lock_guard<std::mutex> l(mu);
+  locked.clear();
+  for (void* p : taken) munmap(p, 8 << 20);
+  taken.clear();
+}
 bool is_locked(const void* p) {
   auto it = locked.upper_bound((const char*)p);
   return it != locked.begin() && (--it, (const char*)p < it->first + it->second);
@@ -59,15 +68,21 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
   std::lock_guard<std::mutex> l(mu);
   if (fail_lock) return cudaErrorMemoryAllocation;
-  *p = malloc(n);
+  *p = mmap(nullptr, 8 << 20, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+  taken.push_back(*p);
   locked[(const char*)*p] = n;
   return cudaSuccess;
 }
 cudaError_t cudaFreeHost(void* p) {
   std::lock_guard<std::mutex> l(mu);
-  locked.erase((const char*)p);
-  free(p);
-  return cudaSuccess;
+  for (size_t k = 0; k < taken.size(); ++k)
+    if (taken[k] == p) {
+      munmap(p, 8 << 20);
+      taken.erase(taken.begin() + k);
+      locked.erase((const char*)p);
+      return cudaSuccess;
+    }
+  return cudaErrorInvalidValue;
 }
 cudaError_t cudaHostRegister(void* p, size_t n, unsigned) {
   std::lock_guard<std::mutex> l(mu);
@@ -190,6 +205,15 @@ void handles() {
   check(copies_right(hostcopy::kMin + 1, 6) && largest == hostcopy::kMin + 1, "a copy without an area, by the driver");
   fail_lock = 0;
 }
+void resets() {
+  check(staged(hostcopy::kMin), "a copy before a device reset");
+  device_reset();
+  check(staged(hostcopy::kMin + 1), "a copy after a device reset");
+  hostcopy::handle_made();
+  device_reset();
+  hostcopy::handle_gone();
+  check(hostcopy::area().mem == nullptr && staged(hostcopy::kMin + 2), "a copy after the area went with a reset");
+}
 void errors() {
   const std::vector<unsigned char> src = pattern(hostcopy::kMin * 2, 7);
   std::vector<unsigned char> dst(src.size());
@@ -220,6 +244,7 @@ int main() {
   sizes();
   threads();
   handles();
+  resets();
   errors();
   no_helpers();
   printf("%d\n", fails);

@@ -1,8 +1,8 @@
 """The threaded copies of large host arrays (koral-zig_b200/csrc/kc_host_copy.cuh) on
 the host, against a stand-in for the runtime calls whose copies run as late as the
 waits allow (host_copy_check.cpp): sizes around the staged minimum and its chunks,
-page-locked arrays, several threads, the area given back and made again, failing
-copies, helper threads that cannot be made."""
+page-locked arrays, several threads, the area given back and made again, device resets,
+failing copies, helper threads that cannot be made."""
 import os
 import shutil
 import subprocess
