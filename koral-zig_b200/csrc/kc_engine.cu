@@ -305,8 +305,11 @@ void launch_set_bc(kc_handle* h) {
   PassScope ps(h, KC_PASS_BC);
   const DGrid& gr = h->gr;
   const long ng = gr.ng;
-  const bool corners = gr.nx > 1 && gr.ny > 1;
-  const long n = !corners ? 0 : gr.nz == 1 ? 4 * 2 * ng : 4L * ((long)gr.nx + gr.ny + gr.nz) * 2 * ng + 8 * ng * ng * ng;
+  // corners lie between two directions that have ghosts (ny = 1 is a plane in x alone)
+  const bool xg = gr.nx > 1;
+  long n = 0;
+  if (gr.ny > 1 && gr.nz > 1) n = 4L * (gr.nx + (xg ? gr.ny + gr.nz : 0)) * 2 * ng + (xg ? 8 * ng * ng * ng : 0);
+  else if (gr.ny > 1 && xg) n = 4 * 2 * ng;
   BcArgs a;
   for (int k = 0; k < 3; ++k) a.bc[k] = h->sp.bc[k];
   a.gam = h->sp.gam;

@@ -603,7 +603,8 @@ __device__ __forceinline__ void edge_task(const DGrid& gr, int pa, int pb, int p
 }
 // 2D: the four corners. 3D: the edges along z, y and x over the domain, and the 8
 // corner cubes (bc.zig:457), copies of the domain's corner cells (the reference's
-// edges also run through the cubes, which then overwrite them).
+// edges also run through the cubes, which then overwrite them). A 3D grid of one
+// cell in x has no ghosts there: only its edges along x.
 __device__ __forceinline__ void corner_task(const DGrid& gr, const int bc[3], long t, GhostTask& g) {
   const long nx = gr.nx, ny = gr.ny, nz = gr.nz, ng = gr.ng, ntask = 2 * ng;
   g.n = 0;
@@ -614,17 +615,18 @@ __device__ __forceinline__ void corner_task(const DGrid& gr, const int bc[3], lo
               bc[1] == KC_BC_PERIODIC, g);
     return;
   }
-  long cc = t / ntask;  // over the 4 nz, 4 ny and 4 nx slices of the three edge groups
-  if (cc < 4 * (nx + ny + nz)) {
+  const long lz = nx > 1 ? nz : 0, ly = nx > 1 ? ny : 0;
+  long cc = t / ntask;  // over the 4 lz, 4 ly and 4 nx slices of the three edge groups
+  if (cc < 4 * (nx + ly + lz)) {
     int pa = 0, pb = 1, pc = 2;
     long len = nz;
-    if (cc >= 4 * nz) {
-      cc -= 4 * nz;
+    if (cc >= 4 * lz) {
+      cc -= 4 * lz;
       pb = 2;
       pc = 1;
       len = ny;
-      if (cc >= 4 * ny) {
-        cc -= 4 * ny;
+      if (cc >= 4 * ly) {
+        cc -= 4 * ly;
         pa = 1;
         pc = 0;
         len = nx;
@@ -633,9 +635,9 @@ __device__ __forceinline__ void corner_task(const DGrid& gr, const int bc[3], lo
     edge_task(gr, pa, pb, pc, cc % len, (int)(cc / len), t % ntask, false, false, g);
     return;
   }
-  t -= 4 * (nx + ny + nz) * ntask;
+  t -= 4 * (nx + ly + lz) * ntask;
   const long per = ng * ng * ng;
-  if (t >= 8 * per) return;
+  if (nx == 1 || t >= 8 * per) return;
   const int cube = (int)(t / per);
   t %= per;
   const bool xh = cube & 1, yh = cube & 2, zh = cube & 4;

@@ -75,6 +75,46 @@ def test_ghost_fill_on_every_boundary(bc, nz):
     _same(gpu, orc)
 
 
+@pytest.mark.parametrize("bc_z", [0, 1])
+def test_ghost_fill_of_a_single_shell(bc_z):
+    """One cell in x: no ghosts there, and the y-z edges filled from the y and z faces
+    (strips copied, means at the first and second diagonal), against plain numpy."""
+    kc = koralcuda()
+    kc.lib()
+    src = kc.Sim(kc.puffy_grid(24, 9, 7), kc.puffy_options())
+    src.initPuffy(1e-3, 1e-3, 5)
+    grid, ng = kc.puffy_grid(1, 9, 7), 3
+    assert grid.ng == ng
+    sim = kc.Sim(grid, kc.puffy_options(bc_y=1, bc_z=bc_z))
+    p = src.p.reshape(7 + 2 * ng, 9 + 2 * ng, 24 + 2 * ng, 13)[:, :, 15].copy()
+    p[:, :, 2] = np.linspace(0.0, 1e-3, p[:, :, 2].size).reshape(p.shape[:2])  # no two cells alike
+    sim.set_prims(p.reshape(-1, 13))
+    sim.set_cons(np.full((p.shape[0] * p.shape[1], 13), np.nan))
+    sim.setBc()
+
+    def y(iy):
+        return iy + ng
+
+    z, want = y, p.copy()
+    for i in range(1, ng + 1):  # faces
+        want[ng:-ng, y(-i)], want[ng:-ng, y(8 + i)] = p[ng:-ng, y(0)], p[ng:-ng, y(8)]
+        want[z(-i), ng:-ng] = p[z(7 - i if bc_z == 0 else 0), ng:-ng]
+        want[z(6 + i), ng:-ng] = p[z(i - 1 if bc_z == 0 else 6), ng:-ng]
+    face, filled = want.copy(), np.zeros(p.shape[:2], bool)
+    for ys, ye in ((-1, 0), (1, 8)):
+        for zs, ze in ((-1, 0), (1, 6)):
+            for k in range(2, ng + 1):
+                want[z(ze + zs), y(ye + k * ys)] = face[z(ze), y(ye + k * ys)]
+                want[z(ze + k * zs), y(ye + ys)] = face[z(ze + k * zs), y(ye)]
+            for k in (1, 2):
+                want[z(ze + k * zs), y(ye + k * ys)] = 0.5 * (face[z(ze), y(ye + k * ys)] + face[z(ze + k * zs), y(ye)])
+            for k in range(1, ng + 1):
+                filled[z(ze + zs), y(ye + k * ys)] = filled[z(ze + k * zs), y(ye + ys)] = True
+            filled[z(ze + 2 * zs), y(ye + 2 * ys)] = True
+    assert np.array_equal(_bits(sim.p), _bits(want.reshape(-1, 13)))
+    assert np.all(np.isfinite(sim.u.reshape(p.shape)[filled]))
+
+
 @pytest.mark.parametrize("shape", [(45, 45, 1), (64, 32, 1), (50, 41, 1), (160, 129, 1), (61, 40, 12)])
 def test_scalar_sums_around_the_fold_sizes(shape):
     """Up to 2048 terms folded by one warp, more in chunks of 1024: 2025, 2048,
