@@ -2,7 +2,8 @@
 // (koral-zig_b200/csrc/kc_implicit_lean.cuh, kc_u2p_lean.cuh) with the plain
 // restatement (include/koral/kimplicit.h, kinvert.h) bit for bit, on the host.
 // Input: cells (geom23, dt, pp), an option variant; prints the number of cells
-// that differ, the number solved and a histogram of the rungs reached.
+// that differ, the number solved and a histogram of the rungs reached. A fourth
+// argument names a file for the plain solve's results (pp, then the six of res).
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -177,6 +178,7 @@ int main(int argc, char** argv) {
   if (variant >= 12) ip.opdamp_maxlevels = 11 - variant;  // a ladder without rungs
   if (variant == 11) ip.convrelerr = 1.0e-12, ip.convrel = 1.0e-13;  // many iterations
   long bad = 0, bad_w = 0, ok = 0, rungs[7] = {0};
+  FILE* results = argc > 4 ? fopen(argv[4], "wb") : nullptr;
   for (long c = 0; c < n; ++c) {
     Geom g;
     geom_from_record(&in[c * 37], g);
@@ -188,6 +190,11 @@ int main(int argc, char** argv) {
     memset(ul, 0, sizeof ul);
     const double* pp00 = &in[c * 37 + 24];
     const ImplicitResult a = solve_implicit_lab(uu, pp, g, dt, gam, rp, op, ip);
+    if (results) {
+      const double r[6] = {(double)a.ok, (double)a.rung, (double)a.iters, (double)a.whichprim, (double)a.whicheq, (double)a.whichframe};
+      fwrite(pp, 8, NV, results);
+      fwrite(r, 8, 6, results);
+    }
     const kc::lean::Warm w = kc::lean::warm_start(pl, g, dt, gam, op, ip);
     double uu0[kc::lean::NU0];
     kc::lean::RefScalars rs;
@@ -249,6 +256,7 @@ int main(int argc, char** argv) {
       if (ra != rb || !same(p1, p2, NV)) ++bad_w;
     }
   }
+  if (results) fclose(results);
   printf("%ld %ld %ld", bad, bad_w, ok);
   for (long x : rungs) printf(" %ld", x);
   printf("\n");

@@ -3,12 +3,14 @@ the implicit and u2p passes around the warp's cell counts, the init's columns wi
 spin, the ordered folds around the chunk size, the ghost fill on every kind of
 boundary; all bit for bit against the oracle."""
 import ctypes
+import subprocess
 
 import numpy as np
 import pytest
 
 from tests.engine import koralcuda
 from tests.orcsim import OracleSim
+from tests.test_lean_solve import cells, lean_binary  # noqa: F401 (fixtures)
 
 pytestmark = pytest.mark.gpu
 
@@ -43,7 +45,7 @@ def test_init_columns_with_spin(spin):
 
 @pytest.mark.parametrize("shape", [(31, 21, 1), (37, 33, 1), (148, 9, 1), (149, 33, 4), (11, 13, 7)])
 def test_steps_at_the_edges_of_the_solve_launches(shape):
-    """651 and 1221 cells (2 and 3 cells a warp), few theta rows, 19668 cells
+    """651 and 1221 cells (2 and 4 cells a warp), few theta rows, 19668 cells
     (full warps, the last one partly filled), and a small grid with faces in
     all three directions (the update's streaming passes by component)."""
     gpu, orc = _pair(*shape)
@@ -137,6 +139,28 @@ def test_batch_forms_agree(n):
     for mode in (1, 3, 5):
         got = kc.implicit_batch(opt, geom, dt, pp, mode=mode)
         assert np.array_equal(_bits(got[0]), _bits(ref[0])) and np.array_equal(got[1], ref[1])
+
+
+@pytest.mark.parametrize("variant,opt", [
+    (1, {"radimp_start_with_bisect": 0}), (2, {"radimp_scale_jacobian": 0}), (3, {"radimp_lag_opac": 1}),
+    (4, {"radimp_allow_rad_ceiling": 0, "radimp_allow_entr_in_4dprim": 0}),
+    (5, {"radimp_opdamp_maxlevels": 1, "radimp_maxiter": 9}), (12, {"radimp_opdamp_maxlevels": -1})])
+def test_batch_options(lean_binary, cells, tmp_path, variant, opt):  # noqa: F811
+    """The batch forms under the options that change the solve's path, lag_opac's
+    own slots among them, against the plain solve on the host (lean_check.cpp's
+    variants)."""
+    path, n = cells
+    out = tmp_path / "plain.bin"
+    subprocess.run([lean_binary, path, str(n), str(variant), str(out)], check=True, capture_output=True)
+    want = np.fromfile(out).reshape(n, 19)
+    kc = koralcuda()
+    kc.lib()
+    a = np.fromfile(path).reshape(n, 37)
+    for mode in (0, 1, 5):
+        pp, res = kc.implicit_batch(kc.puffy_options(**opt), a[:, :23], a[:, 23], a[:, 24:], mode=mode)
+        same = (_bits(pp) == _bits(want[:, :13])) | (np.isnan(pp) & np.isnan(want[:, :13]))
+        assert same.all(), np.argwhere(~same)[:3]
+        assert np.array_equal(res, want[:, 13:].astype(np.int32))
 
 
 def _pairs(sim, cap=8192):
