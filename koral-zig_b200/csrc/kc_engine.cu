@@ -1463,10 +1463,9 @@ int64_t kc_guess_fallbacks(kc_handle* h) {
   return (int64_t)v;
 }
 // The PUFFY init sequence (puffy.zig:873 initAllWith, then initTimestepGuess as
-// problems/puffy/main.zig:304 does). The limotorus profile and the per-cell
-// primitives are built on the host (one torus solve per (x1, x2) column, the
-// cells of a column in parallel threads); set_bc, B from A, the second set_bc
-// and the beta normalization run on the device.
+// problems/puffy/main.zig:304 does), on the device: the limotorus profile by a
+// warp per (x1, x2) column (k_init_columns), the cells' primitives, set_bc, B from
+// A, the second set_bc and the beta normalization.
 int kc_init_puffy(kc_handle* h, double perturb, double perturb_rho, uint64_t seed, double* fac_out) {
   if (!h) return KC_ERR_INVALID_CONFIG;
   const DGrid& gr = h->gr;

@@ -1115,8 +1115,9 @@ __global__ void k_ct_rebuild(DevState s) {
 }
 
 // ---- conserved update + metric source (sim.zig:1140,1542) --------------------
-// Two streaming kernels bound by HBM: u + du of the flux differences, then
-// + dt times the metric source, the reference's two additions in their order.
+// Two streaming kernels: u + du of the flux differences (bound by its divisions),
+// then + dt times the metric source (5.1 TB/s), the reference's two additions in
+// their order.
 // As one kernel the source's 81 loads and two stress tensors left the registers
 // for too few loads in flight: 924 us at 192x180x64, 19 at 32x30, against 717
 // and 9 of the two.
@@ -1404,9 +1405,10 @@ struct StepSrc {
 // `lanes` of each warp's 32 take a cell.
 // Measured on the 192x180x64 wedge, per launch: 5.9 ms with 384 threads, 6.5 with
 // 256 and with 512 (the plain solve in one kernel, warm start included: 20.6 ms).
-// A pass of the 192x180x8 grid executes 298 M warp instructions here and 94 M in
-// the warm start, 847 M before; what is left is dependent FP64 latency (3.3 of
-// 9.4 warp cycles an issue), the trial's spills (1.8) and instruction fetch (1.4).
+// A pass of the 192x180x8 grid executes 300 M warp instructions here and 94 M in
+// the warm start, 847 M before; what is left is dependent FP64 latency (3.2 of
+// some eight warp cycles an issue), loads, spills among them (1.3), and instruction
+// fetch (0.7).
 // Small blocks, which would fill an SM's slots as warps end, are slower (32 or 64
 // threads: 7.4 to 7.7 ms): warps that start together stay in the same part of the
 // code. A barrier a trip over the whole block gains nothing on top (6.3 ms).

@@ -340,7 +340,7 @@ class Sim:
         self._check(self._lib.kc_set_implicit_mode(self._h, mode))
 
     def set_precision(self, mode):
-        """KC_PLAIN_FP64 or KC_MIXED (FP32 reconstruction, LAXF and flux-CT)."""
+        """KC_PLAIN_FP64, KC_MIXED (FP32 LAXF and flux-CT; no faster) or a set of KC_FP32_* pieces."""
         self._check(self._lib.kc_set_precision(self._h, mode))
 
     def scalars(self, dt=0.0, r_lum=5000.0, r_scale=15.0):
